@@ -292,13 +292,7 @@ static int run_yi(RefCtx &c, int inum, int tj, cudaStream_t s)
 {
     const long ntiles = (inum + 31) / 32;
     if (c.fp.Y.ensure(sizeof(double2) * ntiles * 32 * yh_count(tj)) || c.etmp.ensure(sizeof(double) * inum)) return -1;
-    switch (tj) {
-    case 4: return launch_yi<double, 4>(c.model, c.model.yd, c.fp, inum, c.etmp.as<double>(), s);
-    case 6: return launch_yi<double, 6>(c.model, c.model.yd, c.fp, inum, c.etmp.as<double>(), s);
-    case 8: return launch_yi<double, 8>(c.model, c.model.yd, c.fp, inum, c.etmp.as<double>(), s);
-    }
-    set_error("twojmax %d not supported", tj);
-    return -1;
+    return launch_yi_full(tj, c.model.yd, c.fp, inum, c.etmp.as<double>(), nullptr, s);
 }
 
 int ref_snap_ui(double *ur, double *ui, const double *rij, double rcut, double wj, double rfac0, double rmin0,
@@ -371,9 +365,6 @@ int ref_snap_yi(double *yr, double *yi, const double *ur, const double *ui, cons
     return 0;
 }
 
-int launch_yi_pa_d(const SnapModel &m, const YParams<double> &yp, ForcePath &fp, int inum, const double *G,
-                   cudaStream_t s);
-
 // Y with per-atom coefficients beta [jjb][inum] (cpuSnap4.cpp:601-691): the
 // model's coefficients are all 1, so its per-triple factors carry only the
 // multiplicities and the bnorm / (j1+1)/(j+1) scalings
@@ -387,7 +378,7 @@ int ref_snap_yi_beta(double *yr, double *yi, const double *ur, const double *ui,
     if (load_tiles(c, ur, ui, inum, tj, s)) return -1;
     const long ntiles = (inum + 31) / 32;
     if (c.fp.Y.ensure(sizeof(double2) * ntiles * 32 * yh_count(tj))) return -1;
-    if (launch_yi_pa_d(c.model, c.model.yd, c.fp, inum, beta, s)) return -1;
+    if (launch_yi_full(tj, c.model.yd, c.fp, inum, nullptr, beta, s)) return -1;
     const long n = (long)inum * idxu_count(tj);
     k_ytiles_to_ref<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(c.fp.Y.as<double2>(), inum, tj, yh_count(tj), yr, yi);
     MDP_CUDA_TRY(cudaGetLastError());
@@ -709,9 +700,9 @@ int ref_snap_yi_me(double *yr, double *yi, const double *ur, const double *ui, c
 #define MDP_YI_ME(TJ)                                                                                              \
     {                                                                                                              \
         const size_t sm = yi_me_smem_bytes<TJ>();                                                                  \
-        if (kernel_setup((const void *)k_snap_yi_me<TJ>, YiWarps<double, TJ>::n * 32, sm, &per_sm, "k_snap_yi_me")) \
+        if (kernel_setup((const void *)k_snap_yi_me<TJ>, YI_WARPS * 32, sm, &per_sm, "k_snap_yi_me")) \
             return -1;                                                                                             \
-        k_snap_yi_me<TJ><<<std::min(A.ntiles, num_sms() * per_sm), YiWarps<double, TJ>::n * 32, sm, s>>>(          \
+        k_snap_yi_me<TJ><<<std::min(A.ntiles, num_sms() * per_sm), YI_WARPS * 32, sm, s>>>(          \
             Ut, inum, c.model.yd, A, Y);                                                                           \
     }
     switch (tj) {

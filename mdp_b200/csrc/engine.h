@@ -130,6 +130,7 @@ struct DevBuf {
 
 struct ForcePath {
     DevBuf pcount, poff, prij, pinfo, pab, smap, dE, Ut, Y, scan_tmp;
+    DevBuf Ypart, esum;   // few tiles: Y and energy shares of the coupling groups
     DevBuf B, G;   // quadratic SNAP: per-atom bispectrum and coefficients [k][atom]
     DevBuf pcw, elem, ecoef;   // several elements: per-pair cutoff / weight, atom elements, coeffelem
     const int *u_welem = nullptr;     // U stage: element of each atom, for wself per element block
@@ -147,7 +148,11 @@ struct ForcePath {
 // per-stage launchers, one translation unit per (stage, precision)
 template <typename T, int TJ> int launch_ui(const SnapModel &m, ForcePath &fp, int inum, cudaStream_t s);
 template <typename T, int TJ>
-int launch_yi(const SnapModel &m, const YParams<T> &yp, ForcePath &fp, int inum, double *eatom, cudaStream_t s);
+int launch_yi(const YParams<T> &yp, ForcePath &fp, int inum, double *eatom, cudaStream_t s);
+template <int TJ>
+int launch_yi_pa_d(const YParams<double> &yp, ForcePath &fp, int inum, const double *G, cudaStream_t s);
+int launch_yi_full(int tj, const YParams<double> &yp, ForcePath &fp, int inum, double *eatom, const double *G,
+                   cudaStream_t s);
 template <typename T, int TJ> int launch_fi(const SnapModel &m, ForcePath &fp, int inum, int nm, cudaStream_t s);
 
 // One plain-SNAP force evaluation on device data: x (anum, double4, ghosts

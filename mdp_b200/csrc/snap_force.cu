@@ -92,7 +92,8 @@ void DevBuf::release()
 
 void ForcePath::release()
 {
-    DevBuf *b[] = {&pcount, &poff, &prij, &pinfo, &pab, &smap, &dE, &Ut, &Y, &scan_tmp, &B, &G, &pcw, &elem, &ecoef};
+    DevBuf *b[] = {&pcount, &poff, &prij, &pinfo, &pab, &smap, &dE, &Ut, &Y, &Ypart, &esum, &scan_tmp, &B, &G, &pcw,
+                   &elem, &ecoef};
     for (auto x : b) x->release();
     for (auto &e : ev)
         if (e) { cudaEventDestroy(e); e = nullptr; }
@@ -295,8 +296,7 @@ int model_init(SnapModel &m, const mdp_snap_params *p)
         }
         return 0;
     };
-    if (assign(yi_warps(false, tj), m.yd.lay_mb, m.yd.lay_o, m.yd.lay_st) ||
-        assign(yi_warps(true, tj), m.yf.lay_mb, m.yf.lay_o, m.yf.lay_st)) {
+    if (assign(YI_WARPS, m.yd.lay_mb, m.yd.lay_o, m.yd.lay_st)) {
         set_error("Y-kernel warp assignment failed");
         return -1;
     }
@@ -315,14 +315,12 @@ static int launch_snap(const SnapModel &m, const YParams<T> &yp, ForcePath &fp, 
                        double *eatom, cudaStream_t s)
 {
     if (launch_ui<T, TJ>(m, fp, inum, s)) return -1;
-    if (launch_yi<T, TJ>(m, yp, fp, inum, eatom, s)) return -1;
+    if (launch_yi<T, TJ>(yp, fp, inum, eatom, s)) return -1;
     return launch_fi<T, TJ>(m, fp, inum, nm, s);
 }
 
 int launch_bi_tiles(const double2 *Ut, int natoms, int tj, int bnorm, int bzero, double *bout, long bstride,
                     cudaStream_t s);
-int launch_yi_pa_d(const SnapModel &m, const YParams<double> &yp, ForcePath &fp, int inum, const double *G,
-                   cudaStream_t s);
 
 // Quadratic SNAP, one thread per atom: G[k][atom] = beta_k + (Q B)_k (the
 // per-atom coefficients of cpuComputeBeta2, cpuSnap.cpp:1713-1737) and
@@ -365,7 +363,7 @@ static int launch_snap_quad(const SnapModel &m, ForcePath &fp, int inum, int nm,
     k_snap_quad<<<(inum + QUAD_THREADS - 1) / QUAD_THREADS, QUAD_THREADS, 0, s>>>(fp.B.as<double>(), inum, m.quad,
                                                                                fp.G.as<double>(), eatom);
     count_launches(2);
-    if (launch_yi_pa_d(m, m.yq, fp, inum, fp.G.as<double>(), s)) return -1;
+    if (launch_yi_pa_d<TJ>(m.yq, fp, inum, fp.G.as<double>(), s)) return -1;
     return launch_fi<double, TJ>(m, fp, inum, nm, s);
 }
 
@@ -413,9 +411,9 @@ static int launch_snap_me(const SnapModel &m, ForcePath &fp, int inum, int nm, d
     k_snap_ei_me<TJ><<<std::min(A.ntiles, num_sms() * per_sm), BI_WARPS * 32, 0, s>>>(
         fp.Ut.as<double2>(), inum, m.p.bnormflag, A, eatom);
     const size_t sm = yi_me_smem_bytes<TJ>();
-    if (kernel_setup((const void *)k_snap_yi_me<TJ>, YiWarps<double, TJ>::n * 32, sm, &per_sm, "k_snap_yi_me"))
+    if (kernel_setup((const void *)k_snap_yi_me<TJ>, YI_WARPS * 32, sm, &per_sm, "k_snap_yi_me"))
         return -1;
-    k_snap_yi_me<TJ><<<std::min(A.ntiles, num_sms() * per_sm), YiWarps<double, TJ>::n * 32, sm, s>>>(
+    k_snap_yi_me<TJ><<<std::min(A.ntiles, num_sms() * per_sm), YI_WARPS * 32, sm, s>>>(
         fp.Ut.as<double2>(), inum, m.yq, A, fp.Y.as<double2>());
     count_launches(2);
     fp.fr_pcw = fp.pcw.as<double2>();

@@ -5,10 +5,12 @@
 //   k_snap_ui   U_i = sum_j sfac(r_ij) U(r_ij) + wself, mirrored   (:11-244)
 //               one warp per atom, lanes over its pairs, per-row
 //               shared-memory transpose to sum the lanes
-//   k_snap_yi   Y_i = sum_{j1 j2} beta' Z_{j1 j2 j}(U_i)  and
+//   k_snap_y    Y_i = sum_{j1 j2} beta' Z_{j1 j2 j}(U_i)  and
 //               E_i = beta0 + 2/3 sum_half w Re(U* Y)        (:250-421, :697-792)
-//               tiles of 32 atoms (lane = atom), U tile resident in shared
-//               memory, every (j1,j2,j) row of Z specialised at compile time
+//               (y_kernels.cuh)
+//   k_snap_yi   the same for a U that need not have the inversion symmetry (the
+//               stage entry points), FP64: tiles of 32 atoms (lane = atom), U
+//               tile resident in shared memory, every (j1,j2,j) row of Z specialised at compile time
 //               so CG coefficients are constant-bank operands and the U rows
 //               it needs are held in registers
 //   k_snap_fr   dE/dr_ij = 2 sum_half w Re(Y* dU/dr)         (:798-1175)
@@ -28,7 +30,7 @@ struct SnapGeom {
     int switchflag;
 };
 
-// Y-kernel parameters.  Lanes are the 32 atoms of a tile.  Output layers j are
+// Y-kernel parameters (the lay_ tables are those of k_snap_yi).  Lanes are the 32 atoms of a tile.  Output layers j are
 // processed one after another by the whole CTA; within a layer every warp walks
 // the same sequence of (j1, j2) couplings, so the code in flight is one
 // coupling's few kilobytes and stays in the instruction cache.  Each warp owns
@@ -48,40 +50,10 @@ struct YParams {
     // betaY[tri] * G[kmap[tri]] (betaY then holds the multiplicity factors)
     unsigned char kmap[NTRI];
 };
-// warps per Y CTA: FP64 10 (two per row of the costliest layer; 168
-// registers; measured 65 ms at 2M atoms against 70 / 71 / 68 / 68 / 74 ms for
-// 9 / 8 / 11 / 12 / 14 warps; its 146 KB U tile leaves room for one CTA per
-// SM); FP32 8 with two CTAs per SM (92 registers, 93 KB of shared memory
-// each, so one CTA's barrier waits overlap the other's work: the Y stage takes
-// 26.1 ms at 2M atoms against 28.3 / 27.1 / 26.8 / 28.2 ms for 6 / 7 / 10 /
-// 12 warps at two CTAs and 28.4 ms for 20 warps at one).  At 2J <= 4 no layer has more than three rows and the extra
-// warps only wait at the barriers: the FP32 per-atom-coefficient kernel of the
-// surrogate takes 4 (surrogate steps at 2M atoms: 14.8 ms against 14.9 / 15.2
-// / 15.8 / 17.6 / 16.9 ms at 3 / 6 / 8 / 12 / 20 warps; 2 cannot cover the
-// three rows).
-#ifndef YI_W4_D
-#define YI_W4_D 10
-#endif
-#ifndef YI_W4_F
-#define YI_W4_F 4
-#endif
-#ifndef YI_W8_F
-#define YI_W8_F 8
-#endif
-#ifndef YI_MINB_F
-#define YI_MINB_F 2
-#endif
-__host__ __device__ constexpr int yi_warps(bool fp32, int tj)
-{
-    return fp32 ? (tj <= 4 ? YI_W4_F : YI_W8_F) : (tj <= 4 ? YI_W4_D : 10);
-}
-// CTAs per SM the Y kernel is compiled for (register cap)
-template <typename T> __host__ __device__ constexpr int yi_min_blocks()
-{
-    return std::is_same<T, float>::value ? YI_MINB_F : 1;
-}
-template <typename T, int TJ> struct YiWarps { static constexpr int n = yi_warps(false, TJ); };
-template <int TJ> struct YiWarps<float, TJ> { static constexpr int n = yi_warps(true, TJ); };
+// warps per Y CTA: 10 (two per row of the costliest layer; 168 registers; 65 ms
+// at 2M atoms against 70 / 71 / 68 / 68 / 74 ms for 9 / 8 / 11 / 12 / 14 warps;
+// its 146 KB U tile leaves room for one CTA per SM)
+constexpr int YI_WARPS = 10;
 
 __host__ __device__ constexpr bool coupling_ok(int j1, int j2, int j)
 {
@@ -745,73 +717,70 @@ __device__ __forceinline__ void z_rows(const int mb, const int o, const int st,
 
 // all couplings of output layer J, in enumeration order (every warp walks the
 // same sequence, so the code in flight is one coupling's)
-template <typename T, int TJ, bool PA, int J, int J1, int J2>
-__device__ __forceinline__ void z_layer(const int mb, const int o, const int st,
-                                        const typename cplx<T>::type *__restrict__ Us, const int lane,
-                                        const YParams<T> &P, const T *__restrict__ Gs, YRow<T> &acc)
+template <int TJ, bool PA, int J, int J1, int J2>
+__device__ __forceinline__ void z_layer(const int mb, const int o, const int st, const double2 *__restrict__ Us,
+                                        const int lane, const YParams<double> &P, const double *__restrict__ Gs,
+                                        YRow<double> &acc)
 {
     if constexpr (J1 <= TJ) {
         if constexpr (J2 <= J1) {
             if constexpr (coupling_ok(J1, J2, J)) {
                 constexpr int TRI = tri_index(J1, J2, J);
-                T beta = P.betaY[TRI];
+                double beta = P.betaY[TRI];
                 if constexpr (PA) beta *= Gs[P.kmap[TRI] * 32 + lane];
-                z_rows<T, J1, J2, J>(mb, o, st, Us, Us, lane, beta, acc);
+                z_rows<double, J1, J2, J>(mb, o, st, Us, Us, lane, beta, acc);
             }
-            z_layer<T, TJ, PA, J, J1, J2 + 1>(mb, o, st, Us, lane, P, Gs, acc);
+            z_layer<TJ, PA, J, J1, J2 + 1>(mb, o, st, Us, lane, P, Gs, acc);
         } else {
-            z_layer<T, TJ, PA, J, J1 + 1, 0>(mb, o, st, Us, lane, P, Gs, acc);
+            z_layer<TJ, PA, J, J1 + 1, 0>(mb, o, st, Us, lane, P, Gs, acc);
         }
     }
 }
 
 // layer J: each warp builds its partial row, the partials are summed per row,
 // written out (tiled) and folded into the energy identity
-template <typename T, int TJ, int NW, bool PA, int J>
-__device__ __forceinline__ void y_layer(const typename cplx<T>::type *__restrict__ Us,
-                                        typename cplx<T>::type *__restrict__ red,
-                                        typename cplx<T>::type *__restrict__ dst, const int lane, const int w,
-                                        const YParams<T> &P, const T *__restrict__ Gs, double &e)
+template <int TJ, bool PA, int J>
+__device__ __forceinline__ void y_layer(const double2 *__restrict__ Us, double2 *__restrict__ red,
+                                        double2 *__restrict__ dst, const int lane, const int w,
+                                        const YParams<double> &P, const double *__restrict__ Gs, double &e)
 {
-    typedef typename cplx<T>::type T2;
     const int mb = P.lay_mb[J][w];
     if (mb != 255) {
-        YRow<T> acc;
+        YRow<double> acc;
         acc.zero();
-        z_layer<T, TJ, PA, J, 0, 0>(mb, P.lay_o[J][w], P.lay_st[J][w], Us, lane, P, Gs, acc);
+        z_layer<TJ, PA, J, 0, 0>(mb, P.lay_o[J][w], P.lay_st[J][w], Us, lane, P, Gs, acc);
 #pragma unroll
         for (int ma = 0; ma <= J; ma++) red[(w * JD + ma) * 32 + lane] = acc.get(ma);
     }
     __syncthreads();
     constexpr int NE = (J / 2 + 1) * (J + 1);
-    for (int k = w; k < NE; k += NW) {
+    for (int k = w; k < NE; k += YI_WARPS) {
         const int rmb = k / (J + 1), ma = k - rmb * (J + 1);
-        T yr = T(0), yi = T(0);
+        double yr = 0.0, yi = 0.0;
 #pragma unroll
-        for (int v = 0; v < NW; v++)
+        for (int v = 0; v < YI_WARPS; v++)
             if (P.lay_mb[J][v] == rmb) {
-                const T2 t = red[(v * JD + ma) * 32 + lane];
+                const double2 t = red[(v * JD + ma) * 32 + lane];
                 yr += t.x; yi += t.y;
             }
         if constexpr (!PA) {
-            const T2 u = Us[(idxu_block(J) + k) * 32 + lane];
+            const double2 u = Us[(idxu_block(J) + k) * 32 + lane];
             const double wgt = (2 * rmb < J) ? 1.0 : (ma < rmb ? 1.0 : (ma == rmb ? 0.5 : 0.0));
-            e += wgt * ((double)u.x * (double)yr + (double)u.y * (double)yi);
+            e += wgt * (u.x * yr + u.y * yi);
         }
-        dst[(yh_block(J) + k) * 32 + lane] = T2{yr, yi};
+        dst[(yh_block(J) + k) * 32 + lane] = double2{yr, yi};
     }
     __syncthreads();
 }
 
-template <typename T, int TJ, int NW, bool PA, int J>
-__device__ __forceinline__ void y_all(const typename cplx<T>::type *__restrict__ Us,
-                                      typename cplx<T>::type *__restrict__ red,
-                                      typename cplx<T>::type *__restrict__ dst, const int lane, const int w,
-                                      const YParams<T> &P, const T *__restrict__ Gs, double &e)
+template <int TJ, bool PA, int J>
+__device__ __forceinline__ void y_all(const double2 *__restrict__ Us, double2 *__restrict__ red,
+                                      double2 *__restrict__ dst, const int lane, const int w,
+                                      const YParams<double> &P, const double *__restrict__ Gs, double &e)
 {
     if constexpr (J >= 0) {
-        y_layer<T, TJ, NW, PA, J>(Us, red, dst, lane, w, P, Gs, e);
-        y_all<T, TJ, NW, PA, J - 1>(Us, red, dst, lane, w, P, Gs, e);
+        y_layer<TJ, PA, J>(Us, red, dst, lane, w, P, Gs, e);
+        y_all<TJ, PA, J - 1>(Us, red, dst, lane, w, P, Gs, e);
     }
 }
 
@@ -826,46 +795,44 @@ __host__ __device__ constexpr int nbispec(int tj)
     return n;
 }
 
-template <typename T, int TJ, bool PA = false>
+template <int TJ, bool PA>
 constexpr size_t yi_smem_bytes()
 {
-    return (size_t)idxu_count(TJ) * 32 * sizeof(typename cplx<T>::type) +
-           (size_t)YiWarps<T, TJ>::n * JD * 32 * sizeof(typename cplx<T>::type) + YiWarps<T, TJ>::n * 32 * sizeof(double) +
-           (PA ? (size_t)nbispec(TJ) * 32 * sizeof(T) : 0);
+    return (size_t)idxu_count(TJ) * 32 * sizeof(double2) + (size_t)YI_WARPS * JD * 32 * sizeof(double2) +
+           YI_WARPS * 32 * sizeof(double) + (PA ? (size_t)nbispec(TJ) * 32 * sizeof(double) : 0);
 }
 
 // Output Y in 32-atom tiles: Y[tile][k][lane], k = half-plane index.
 // PA: per-atom coefficients G[k * natoms + atom] (k over the nbispec(TJ)
 // components) instead of the model's; no energy is written.
-template <typename T, int TJ, bool PA = false>
-__global__ void __launch_bounds__(YiWarps<T, TJ>::n * 32, yi_min_blocks<T>())
-k_snap_yi(const typename cplx<T>::type *__restrict__ Ut, int natoms, const __grid_constant__ YParams<T> P,
-          typename cplx<T>::type *__restrict__ Y, double *__restrict__ eatom, const T *__restrict__ G = nullptr)
+template <int TJ, bool PA>
+__global__ void __launch_bounds__(YI_WARPS * 32, 1)
+k_snap_yi(const double2 *__restrict__ Ut, int natoms, const __grid_constant__ YParams<double> P,
+          double2 *__restrict__ Y, double *__restrict__ eatom, const double *__restrict__ G)
 {
-    typedef typename cplx<T>::type T2;
-    constexpr int NW = YiWarps<T, TJ>::n;
+    constexpr int NW = YI_WARPS;
     constexpr int NU = idxu_count(TJ);
     constexpr int NYH = yh_count(TJ);
     constexpr int NK = nbispec(TJ);
     extern __shared__ __align__(16) unsigned char smraw[];
-    T2 *Us = reinterpret_cast<T2 *>(smraw);
-    T2 *red = Us + NU * 32;                                // [warp][ma][lane]
+    double2 *Us = reinterpret_cast<double2 *>(smraw);
+    double2 *red = Us + NU * 32;                                // [warp][ma][lane]
     double *ered = reinterpret_cast<double *>(red + NW * JD * 32);
-    T *Gs = reinterpret_cast<T *>(ered + NW * 32);         // [k][lane] (PA)
+    double *Gs = ered + NW * 32;                                // [k][lane] (PA)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int ntiles = (natoms + 31) >> 5;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const T2 *src = Ut + (size_t)tile * NU * 32;
+        const double2 *src = Ut + (size_t)tile * NU * 32;
         for (int k = threadIdx.x; k < NU * 32; k += NW * 32) Us[k] = src[k];
         if constexpr (PA) {
             for (int k = threadIdx.x; k < NK * 32; k += NW * 32) {
                 const int a = tile * 32 + (k & 31);
-                Gs[k] = (a < natoms) ? G[(size_t)(k >> 5) * natoms + a] : T(0);
+                Gs[k] = (a < natoms) ? G[(size_t)(k >> 5) * natoms + a] : 0.0;
             }
         }
         __syncthreads();
         double e = 0.0;
-        y_all<T, TJ, NW, PA, TJ>(Us, red, Y + (size_t)tile * NYH * 32, lane, w, P, Gs, e);
+        y_all<TJ, PA, TJ>(Us, red, Y + (size_t)tile * NYH * 32, lane, w, P, Gs, e);
         if constexpr (PA) {
             __syncthreads();
             continue;
@@ -1103,15 +1070,15 @@ __device__ __forceinline__ void y_all_me(const double2 *__restrict__ Ut, const i
 template <int TJ>
 constexpr size_t yi_me_smem_bytes()
 {
-    return (size_t)YiWarps<double, TJ>::n * JD * 32 * sizeof(double2);
+    return (size_t)YI_WARPS * JD * 32 * sizeof(double2);
 }
 
 template <int TJ>
-__global__ void __launch_bounds__(YiWarps<double, TJ>::n * 32, 1)
+__global__ void __launch_bounds__(YI_WARPS * 32, 1)
 k_snap_yi_me(const double2 *__restrict__ Ut, int natoms, const __grid_constant__ YParams<double> P,
              const __grid_constant__ MeArgs A, double2 *__restrict__ Y)
 {
-    constexpr int NW = YiWarps<double, TJ>::n;
+    constexpr int NW = YI_WARPS;
     extern __shared__ __align__(16) unsigned char smraw[];
     double2 *red = reinterpret_cast<double2 *>(smraw);   // [warp][ma][lane]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
