@@ -1,24 +1,29 @@
-// U stage launchers (k_snap_uc), all precisions.
-#include "engine.h"
-
-#include <algorithm>
+// U stage launchers (k_snap_ur), all precisions.
+#include "u_kernels.cuh"
 
 namespace mdp {
 
-template <typename T, int TJ>
-int launch_ui(const SnapModel &m, ForcePath &fp, int inum, cudaStream_t s)
+template <typename T, int TJ, int SPL>
+static void launch_ur(ForcePath &fp, int inum, cudaStream_t s)
 {
-    typedef typename cplx<T>::type T2;
+    const int atoms = (inum + 31) & ~31, per_cta = UR_WARPS * 32 / SPL;
+    const int grid = (atoms + per_cta - 1) / per_cta * UrJobs<T, TJ>::n;
+    k_snap_ur<T, TJ, SPL><<<grid, UR_WARPS * 32, 0, s>>>(fp.poff.as<int>(), fp.prij.as<double4>(),
+                                                         fp.pab.as<double4>(), inum,
+                                                         fp.Ut.as<typename cplx<T>::type>(), fp.u_welem, fp.u_ipad);
+}
+
+// Four lanes share an atom's pairs while one warp per (tile, job) would leave
+// schedulers without a warp: the walk over about 20 pairs is then what takes
+// the time (FP64, 2J = 8: 128 atoms 19 -> 11 us, 2,000 atoms 24 -> 17 us; at
+// 16,000 atoms the lanes' common sums make it 69 -> 72 us).
+template <typename T, int TJ>
+int launch_ui(const SnapModel &, ForcePath &fp, int inum, cudaStream_t s)
+{
     if (tu_ensure_tables()) return -1;
-    const size_t sm = uc_smem_bytes<T, TJ>();
-    int per_sm = 0;
-    if (kernel_setup((const void *)k_snap_uc<T, TJ>, uc_warps<T, TJ>() * 32, sm, &per_sm, "k_snap_uc")) return -1;
-    const int ntiles = (inum + 31) / 32;
-    const int blocks = std::min(ntiles, num_sms() * per_sm);
     if (fp.timing) cudaEventRecord(fp.ev[1], s);
-    k_snap_uc<T, TJ><<<blocks, uc_warps<T, TJ>() * 32, sm, s>>>(fp.poff.as<int>(), fp.prij.as<double4>(),
-                                                             fp.pab.as<double4>(), inum, fp.Ut.as<T2>(),
-                                                             fp.u_welem, fp.u_ipad);
+    if ((inum + 31) / 32 * UrJobs<T, TJ>::n <= 4 * num_sms()) launch_ur<T, TJ, 4>(fp, inum, s);
+    else launch_ur<T, TJ, 1>(fp, inum, s);
     return 0;
 }
 

@@ -329,63 +329,8 @@ __device__ __forceinline__ void cf_fwd(const T ar, const T ai, const T br, const
     }
 }
 
-// ---------------------------------------------------------------------------
-// k_snap_uc: U of a 32-atom tile, one warp per column of the half plane.
-//
-// Lane = atom.  Each lane walks its own atom's pairs, uc_pb<T>() per pass, and
-// per pair recomputes the recursion path that reaches its warp's column: the
-// seed chain (rows 1, 2c..2c+1 of the columns c below, each mirrored into the
-// next column's seed) and then the column's own rows, which it adds into a
-// half-plane tile in shared memory ([uh index][lane]).  Every column's path
-// has one row per layer 1..TJ, so the warps' work is equal; the top two
-// columns share the last warp (the top one continues from the row the other
-// ends its chain with).  Warps own disjoint tile entries: no atomics.  The
-// tile is then written out as the full plane with wself on the diagonal,
-// and rows mb > j/2 and the middle rows' right halves by inversion symmetry
-// (cpuSnap4.cpp:11-244, cpuAddWself2Ui).
-// (a, b, sfac) of each pair come from the pair stage.
-// ---------------------------------------------------------------------------
-// pairs per lane per pass: FP32 takes two (independent chains, half the tile
-// updates; 8.1 against 8.2 ms at 2M atoms); FP64 one (two measured 18.1
-// against 15.7 ms: twice the unrolled code per warp path; with the split
-// plan, 19.9 ms at two CTAs per SM and 21.8 ms at three against 15.1 ms)
-#ifndef UC_PB_D
-#define UC_PB_D 1
-#endif
-template <typename T> __host__ __device__ constexpr int uc_pb() { return std::is_same<T, float>::value ? 2 : UC_PB_D; }
-// Work plan.  One warp per column (the top two columns share the last warp),
-// or, for FP64 at 2J = 8, eight jobs (column, first layer added into the
-// tile, last layer): a job steps through its column's rows below its first
-// layer without adding them, so the deep columns are split across two warps
-// and twice the warps share the tile (U 15.3 against 16.1 ms per step at 2M
-// atoms).  FP32, with two pairs per pass, lost by it (12.0 against 8.3 ms).
-#ifndef UC_SPLIT
-#define UC_SPLIT 1
-#endif
-struct UcJob {
-    int mb, jlo, jhi;
-};
-template <typename T, int TJ> __host__ __device__ constexpr bool uc_split()
-{
-    return UC_SPLIT && TJ == 8 && std::is_same<T, double>::value;
-}
-template <typename T, int TJ> __host__ __device__ constexpr int uc_warps() { return uc_split<T, TJ>() ? 8 : TJ / 2; }
-// CTAs per SM the split FP64 kernel is compiled for: three 74 KB tiles fit an
-// SM's shared memory, which holds 80 registers a thread
-#ifndef UC_MINB_D
-#define UC_MINB_D 3
-#endif
-// (0, the others: no bound, as an explicit 1 makes ptxas spend registers)
-template <typename T, int TJ> __host__ __device__ constexpr int uc_minb() { return uc_split<T, TJ>() ? UC_MINB_D : 0; }
-template <int TJ> __host__ __device__ constexpr UcJob uc_job(int w)
-{
-    constexpr UcJob plan8[8] = {{0, 0, 5}, {0, 6, 8}, {1, 0, 6}, {1, 7, 8},
-                                {2, 0, 6}, {2, 7, 8}, {3, 0, 8}, {4, 0, 8}};
-    return plan8[w];
-}
-// The tile holds the half plane without the entries right of a middle row's
-// centre (the mirror of its left half): 145 entries at 2J = 8 against 155,
-// which lets three FP64 CTAs share an SM (74 KB each) instead of two.
+// the half plane without the entries right of a middle row's centre (the mirror
+// of its left half): 145 entries at 2J = 8 against 155
 __host__ __device__ constexpr int uh_len(int j) { return (j + 1) * ((j + 1) / 2) + (j % 2 == 0 ? j / 2 + 1 : 0); }
 __host__ __device__ constexpr int uh_block(int j)
 {
@@ -394,193 +339,6 @@ __host__ __device__ constexpr int uh_block(int j)
     return n;
 }
 __host__ __device__ constexpr int uh_count(int tj) { return uh_block(tj + 1); }
-template <typename T, int TJ> constexpr size_t uc_smem_bytes()
-{
-    return (size_t)uh_count(TJ) * 32 * sizeof(typename cplx<T>::type);
-}
-
-// per-pair state; the root of the recursion is v_0 = sfac, so every row comes
-// out weighted by sfac (the recursion is linear in its root)
-template <typename T, int TJ>
-struct UcPairs {
-    static constexpr int PB = uc_pb<T>();
-    T ar[PB], ai[PB], br[PB], bi[PB];
-    T pr[PB][TJ + 1], pi[PB][TJ + 1];
-};
-
-// seed chain up to column MB: column C's last chain row (2C+1) mirrored into
-// column C+1's seed, for C = 0..MB-1
-template <typename T, int TJ, int MB, int C>
-__device__ __forceinline__ void uc_chain(UcPairs<T, TJ> &s)
-{
-    if constexpr (C < MB) {
-        constexpr int J = 2 * C + 1;
-#pragma unroll
-        for (int q = 0; q < UcPairs<T, TJ>::PB; q++) {
-            if constexpr (C > 0) cf_fwd<T, TJ, 2 * C, C>(s.ar[q], s.ai[q], s.br[q], s.bi[q], s.pr[q], s.pi[q]);
-            cf_fwd<T, TJ, J, C>(s.ar[q], s.ai[q], s.br[q], s.bi[q], s.pr[q], s.pi[q]);
-            T nr[J + 1], ni[J + 1];
-#pragma unroll
-            for (int ma = 0; ma <= J; ma++) {
-                const T sg = ((C + ma) & 1) ? T(-1) : T(1);
-                nr[J - ma] = sg * s.pr[q][ma]; ni[J - ma] = -sg * s.pi[q][ma];
-            }
-#pragma unroll
-            for (int ma = 0; ma <= J; ma++) { s.pr[q][ma] = nr[ma]; s.pi[q][ma] = ni[ma]; }
-        }
-        uc_chain<T, TJ, MB, C + 1>(s);
-    }
-}
-
-// rows J..JEND of column MB (row J's parent in s.pr/pi), each from layer
-// JACC on added into the tile
-template <typename T, int TJ, int MB, int J, int JEND, int JACC = 0>
-__device__ __forceinline__ void uc_column(UcPairs<T, TJ> &s, typename cplx<T>::type *__restrict__ acc)
-{
-    typedef typename cplx<T>::type T2;
-    if constexpr (J <= JEND) {
-        if constexpr (J > 0) {
-#pragma unroll
-            for (int q = 0; q < UcPairs<T, TJ>::PB; q++)
-                cf_fwd<T, TJ, J, MB>(s.ar[q], s.ai[q], s.br[q], s.bi[q], s.pr[q], s.pi[q]);
-        }
-        if constexpr (J < JACC) {
-            uc_column<T, TJ, MB, J + 1, JEND, JACC>(s, acc);
-            return;
-        }
-        T2 *row = acc + (uh_block(J) + (J + 1) * MB) * 32;
-        constexpr int MAMAX = (2 * MB == J) ? MB : J;
-#pragma unroll
-        for (int ma = 0; ma <= MAMAX; ma++) {
-            const T nu = unorm<T>(J, MB, ma);
-            T2 v = row[ma * 32];
-#pragma unroll
-            for (int q = 0; q < UcPairs<T, TJ>::PB; q++) {
-                if constexpr (std::is_same<T, float>::value)
-                    v = __ffma2_rn(make_float2(nu, nu), make_float2(s.pr[q][ma], s.pi[q][ma]), v);
-                else { v.x += nu * s.pr[q][ma]; v.y += nu * s.pi[q][ma]; }
-            }
-            row[ma * 32] = v;
-        }
-        uc_column<T, TJ, MB, J + 1, JEND, JACC>(s, acc);
-    }
-}
-
-// the work of warp MB: column MB (and, for the last warp, column MB+1)
-template <typename T, int TJ, int MB>
-__device__ __forceinline__ void uc_path(UcPairs<T, TJ> &s, typename cplx<T>::type *__restrict__ acc)
-{
-    uc_chain<T, TJ, MB, 0>(s);
-    if constexpr (MB + 1 < uc_warps<T, TJ>()) {
-        uc_column<T, TJ, MB, (MB == 0 ? 0 : 2 * MB), TJ>(s, acc);
-    } else {
-        // last warp: column MB up to its row 2MB+1, mirror to the seed of
-        // column MB+1 = TJ/2, then column MB's remaining rows continue from a
-        // copy while column TJ/2 takes its single row TJ
-        constexpr int MT = MB + 1;
-        uc_column<T, TJ, MB, (MB == 0 ? 0 : 2 * MB), 2 * MB + 1>(s, acc);
-        T kr[UcPairs<T, TJ>::PB][TJ + 1], ki[UcPairs<T, TJ>::PB][TJ + 1];
-#pragma unroll
-        for (int q = 0; q < UcPairs<T, TJ>::PB; q++)
-#pragma unroll
-            for (int ma = 0; ma <= 2 * MB + 1; ma++) { kr[q][ma] = s.pr[q][ma]; ki[q][ma] = s.pi[q][ma]; }
-        uc_column<T, TJ, MB, 2 * MB + 2, TJ>(s, acc);
-#pragma unroll
-        for (int q = 0; q < UcPairs<T, TJ>::PB; q++) {
-            constexpr int J = 2 * MB + 1;
-#pragma unroll
-            for (int ma = 0; ma <= J; ma++) {
-                const T sg = ((MB + ma) & 1) ? T(-1) : T(1);
-                s.pr[q][J - ma] = sg * kr[q][ma]; s.pi[q][J - ma] = -sg * ki[q][ma];
-            }
-        }
-        uc_column<T, TJ, MT, 2 * MT, TJ>(s, acc);
-    }
-}
-
-template <typename T, int TJ, int MB>
-__device__ __forceinline__ void uc_dispatch(const int w, UcPairs<T, TJ> &s, typename cplx<T>::type *__restrict__ acc)
-{
-    if constexpr (uc_split<T, TJ>()) {
-        if constexpr (MB < uc_warps<T, TJ>()) {
-            constexpr UcJob jb = uc_job<TJ>(MB);
-            if (w == MB) {
-                uc_chain<T, TJ, jb.mb, 0>(s);
-                uc_column<T, TJ, jb.mb, (jb.mb == 0 ? 0 : 2 * jb.mb), jb.jhi, jb.jlo>(s, acc);
-            } else {
-                uc_dispatch<T, TJ, MB + 1>(w, s, acc);
-            }
-        }
-    } else if constexpr (MB < uc_warps<T, TJ>()) {
-        if (w == MB) uc_path<T, TJ, MB>(s, acc);
-        else uc_dispatch<T, TJ, MB + 1>(w, s, acc);
-    }
-}
-
-template <typename T, int TJ>
-__global__ void __launch_bounds__(uc_warps<T, TJ>() * 32, uc_minb<T, TJ>())
-k_snap_uc(const int *__restrict__ poff, const double4 *__restrict__ prij, const double4 *__restrict__ pab,
-          int natoms, typename cplx<T>::type *__restrict__ Ut, const int *__restrict__ welem = nullptr,
-          int ipad = 0)
-{
-    typedef typename cplx<T>::type T2;
-    constexpr int NW = uc_warps<T, TJ>();
-    constexpr int NU = idxu_count(TJ), NUH = uh_count(TJ);
-    extern __shared__ __align__(16) unsigned char smraw[];
-    T2 *acc = reinterpret_cast<T2 *>(smraw);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int ntiles = (natoms + 31) >> 5;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        for (int k = threadIdx.x; k < NUH * 32; k += NW * 32) acc[k] = T2{T(0), T(0)};
-        __syncthreads();
-        const int i = tile * 32 + lane;
-        int p = 0, pend = 0;
-        if (i < natoms) { p = poff[i]; pend = poff[i + 1]; }
-        for (; p < pend; p += UcPairs<T, TJ>::PB) {
-            UcPairs<T, TJ> s;
-#pragma unroll
-            for (int q = 0; q < UcPairs<T, TJ>::PB; q++) {
-                const bool ok = p + q < pend;
-                const double4 g = ok ? pab[p + q] : make_double4(1.0, 0.0, 0.0, 0.0);
-                s.ar[q] = (T)g.x; s.ai[q] = (T)g.y; s.br[q] = (T)g.z; s.bi[q] = (T)g.w;
-                s.pr[q][0] = ok ? (T)prij[p + q].w : T(0);   // v_0 = sfac
-                s.pi[q][0] = T(0);
-            }
-            uc_dispatch<T, TJ, 0>(w, s, acc + lane);
-        }
-        __syncthreads();
-        // full plane out: wself on the diagonal, rows mb > j/2 mirrored.  With
-        // welem (element blocks of virtual atoms v = b * ipad + atom), wself
-        // goes to the atom's own element block only (cpuAddWself2Ui,
-        // cpuSnap4.cpp:193-244, chemflag without wselfallflag).
-        T2 *dst = Ut + (size_t)tile * NU * 32;
-        for (int e = threadIdx.x; e < NU * 32; e += NW * 32) {
-            const int k = e >> 5, l = e & 31;
-            T ws = T(1);
-            if (welem) {
-                const int v = tile * 32 + l;
-                ws = (welem[v % ipad] == v / ipad) ? T(1) : T(0);
-            }
-            int j = 0;
-            while (idxu_block(j + 1) <= k) j++;
-            const int rem = k - idxu_block(j), mb = rem / (j + 1), ma = rem - mb * (j + 1);
-            T2 v;
-            if (2 * mb < j || (2 * mb == j && ma <= mb)) {
-                v = acc[(uh_block(j) + rem) * 32 + l];
-                if (ma == mb) v.x += ws;
-            } else {
-                // mirror: rows mb > j/2 and a middle row's right half
-                const int sb = j - mb, sa = j - ma;
-                const T2 u = acc[(uh_block(j) + (j + 1) * sb + sa) * 32 + l];
-                const T sg = ((sa + sb) & 1) ? T(-1) : T(1);
-                v = T2{sg * (u.x + (sa == sb ? ws : T(0))), -sg * u.y};
-            }
-            dst[e] = v;
-        }
-        __syncthreads();
-    }
-}
-
 // ---------------------------------------------------------------------------
 // k_snap_yi
 // ---------------------------------------------------------------------------
@@ -1159,7 +917,7 @@ template <> struct FAccSel<float> { typedef FAccComp type; };
 //     dF/d(ar + i ai) += A_ma conj(l[ma]) p[ma]        (as (re, im) pairs)
 //     dF/d(br + i bi) -= B_ma conj(l[ma]) p[ma-1]
 // and F itself is the real part of the adjoint of the root u_0 = 1.  In FP32
-// the rows are instead the coefficient-free ones of k_snap_uc (u = unorm v,
+// the rows are instead the coefficient-free ones of k_snap_ur (u = unorm v,
 // A = B = 1, adjoint seeded with unorm Y), which saves the rootpq products.
 // This is about 5,100 operations per pair at 2J=8 against about 14,000 for
 // carrying the three derivative directions forward through the recursion,
@@ -1243,7 +1001,7 @@ __device__ __forceinline__ void fr_fwd(const T ar, const T ai, const T br, const
 }
 
 // FP64 runs the recursion in u-space (rootpq factors), FP32 in the
-// coefficient-free v-space of k_snap_uc (u = unorm v).  Both give the same
+// coefficient-free v-space of k_snap_ur (u = unorm v).  Both give the same
 // gradient; in FP64 the coefficient-free form issues fewer instructions but,
 // at 254 registers, measured twice as slow (its memory latency is exposed).
 template <typename T> __host__ __device__ constexpr bool fr_cf() { return std::is_same<T, float>::value; }
