@@ -909,19 +909,19 @@ template <> struct FAccSel<float> { typedef FAccComp type; };
 //
 // With F(a, b) = sum_half w Re(Y* u(a, b)) (the same half-plane sum as the
 // forward-mode kernel), dE/dx_k = 2 (dsfac u_k F + sfac dF/dx_k) and
-// dF/dx_k = grad_(ar,ai,br,bi) F . d(a,b)/dx_k.  Each U row (layer J, column
-// mb) is n[ma] = A_ma conj(a) p[ma] - B_ma conj(b) p[ma-1] of its parent row p
-// (layer J-1), A_ma = rootpq(J-ma, J-mb), B_ma = rootpq(ma, J-mb).  Its
-// adjoint, for an adjoint row l of layer J, is
-//     l'[k] = A_k a l[k] - B_(k+1) b l[k+1]           (parent row's adjoint)
-//     dF/d(ar + i ai) += A_ma conj(l[ma]) p[ma]        (as (re, im) pairs)
-//     dF/d(br + i bi) -= B_ma conj(l[ma]) p[ma-1]
-// and F itself is the real part of the adjoint of the root u_0 = 1.  In FP32
-// the rows are instead the coefficient-free ones of k_snap_ur (u = unorm v,
-// A = B = 1, adjoint seeded with unorm Y), which saves the rootpq products.
-// This is about 5,100 operations per pair at 2J=8 against about 14,000 for
-// carrying the three derivative directions forward through the recursion,
-// which is how cpuSnap4.cpp:798-1175 computes dU/dr.
+// dF/dx_k = grad_(ar,ai,br,bi) F . d(a,b)/dx_k.  The rows are the
+// coefficient-free ones of k_snap_ur (u = unorm v): a row (layer J, column mb)
+// is n[ma] = conj(a) p[ma] - conj(b) p[ma-1] of its parent row p (layer J-1).
+// Its adjoint, for an adjoint row l of layer J (seeded with unorm Y), is
+//     l'[k] = a l[k] - b l[k+1]                    (parent row's adjoint)
+//     dF/d(ar + i ai) += conj(l[ma]) p[ma]         (as (re, im) pairs)
+//     dF/d(br + i bi) -= conj(l[ma]) p[ma-1]
+// and F itself is the real part of the adjoint of the root u_0 = 1.  This is
+// about 3,900 operations per pair at 2J=8 against about 14,000 for carrying the
+// three derivative directions forward through the recursion, which is how
+// cpuSnap4.cpp:798-1175 computes dU/dr.  (With the normalisation in the rows,
+// rootpq factors on every term, the FP64 kernel took 8.72 ns per atom at
+// 250,000 atoms against 7.69.)
 //
 // Columns mb depend on each other only through the seed rows (the parent of
 // row (2mb, mb) is the mirror of row (2mb-1, mb-1)), so the pass is:
@@ -966,53 +966,6 @@ struct FrState {
     T lr[TJ + 1], li[TJ + 1];                   // adjoint row
 };
 
-// row J-1 -> row J of column MB, in place (entries 0..J), as u_rows does (u-space, rootpq factors)
-template <typename T, int TJ, int J, int MB>
-__device__ __forceinline__ void fr_fwd(const T ar, const T ai, const T br, const T bi, T (&pr)[TJ + 1],
-                                       T (&pi)[TJ + 1])
-{
-    {
-        const T rp = rootpq<T>(J, J - MB);
-        const T nr = -rp * (br * pr[J - 1] + bi * pi[J - 1]);
-        const T ni = -rp * (br * pi[J - 1] - bi * pr[J - 1]);
-        pr[J] = nr; pi[J] = ni;
-    }
-#pragma unroll
-    for (int ma = J - 1; ma >= 1; ma--) {
-        const T rpa = rootpq<T>(J - ma, J - MB), rpb = rootpq<T>(ma, J - MB);
-        const T nr = rpa * (ar * pr[ma] + ai * pi[ma]) - rpb * (br * pr[ma - 1] + bi * pi[ma - 1]);
-        const T ni = rpa * (ar * pi[ma] - ai * pr[ma]) - rpb * (br * pi[ma - 1] - bi * pr[ma - 1]);
-        pr[ma] = nr; pi[ma] = ni;
-    }
-    {
-        const T rpa = rootpq<T>(J, J - MB);
-        const T nr = rpa * (ar * pr[0] + ai * pi[0]);
-        const T ni = rpa * (ar * pi[0] - ai * pr[0]);
-        pr[0] = nr; pi[0] = ni;
-    }
-    if constexpr (MB > 0 && J == 2 * MB) {
-#pragma unroll
-        for (int ma = 0; ma <= MB; ma++) {
-            const T s = (ma & 1) ? T(-1) : T(1);
-            pr[MB + ma] = s * pr[MB - ma];
-            pi[MB + ma] = -s * pi[MB - ma];
-        }
-    }
-}
-
-// FP64 runs the recursion in u-space (rootpq factors), FP32 in the
-// coefficient-free v-space of k_snap_ur (u = unorm v).  Both give the same
-// gradient; in FP64 the coefficient-free form issues fewer instructions but,
-// at 254 registers, measured twice as slow (its memory latency is exposed).
-template <typename T> __host__ __device__ constexpr bool fr_cf() { return std::is_same<T, float>::value; }
-template <typename T, int TJ, int J, int MB>
-__device__ __forceinline__ void fr_row(const T ar, const T ai, const T br, const T bi, T (&pr)[TJ + 1],
-                                       T (&pi)[TJ + 1])
-{
-    if constexpr (fr_cf<T>()) cf_fwd<T, TJ, J, MB>(ar, ai, br, bi, pr, pi);
-    else fr_fwd<T, TJ, J, MB>(ar, ai, br, bi, pr, pi);
-}
-
 // seed S_(MB+1)[J - ma] = (-1)^(MB+ma) conj(row (J = 2MB+1, MB)[ma])
 template <typename T, int TJ, int MB>
 __device__ __forceinline__ void fr_put_seed(const T (&pr)[TJ + 1], const T (&pi)[TJ + 1], T *__restrict__ qs)
@@ -1034,11 +987,11 @@ __device__ __forceinline__ void fr_seeds(const T ar, const T ai, const T br, con
     if constexpr (2 * (MB + 1) <= TJ) {
         if constexpr (MB == 0) {
             pr[0] = T(1); pi[0] = T(0);
-            fr_row<T, TJ, 1, 0>(ar, ai, br, bi, pr, pi);
+            cf_fwd<T, TJ, 1, 0>(ar, ai, br, bi, pr, pi);
         } else {
             // pr/pi hold S_MB (entries 0..2MB-1)
-            fr_row<T, TJ, 2 * MB, MB>(ar, ai, br, bi, pr, pi);
-            fr_row<T, TJ, 2 * MB + 1, MB>(ar, ai, br, bi, pr, pi);
+            cf_fwd<T, TJ, 2 * MB, MB>(ar, ai, br, bi, pr, pi);
+            cf_fwd<T, TJ, 2 * MB + 1, MB>(ar, ai, br, bi, pr, pi);
         }
         fr_put_seed<T, TJ, MB>(pr, pi, qs);
         // the next column starts from the seed just written
@@ -1060,7 +1013,7 @@ template <typename T, int TJ, int J, int MB>
 __device__ __forceinline__ void fr_col_fwd(FrState<T, TJ> &st, T (&pr)[TJ + 1], T (&pi)[TJ + 1])
 {
     if constexpr (J < TJ) {
-        fr_row<T, TJ, J, MB>(st.ar, st.ai, st.br, st.bi, pr, pi);
+        cf_fwd<T, TJ, J, MB>(st.ar, st.ai, st.br, st.bi, pr, pi);
 #pragma unroll
         for (int ma = 0; ma <= J; ma++) { st.ur[fr_row_off(J) + ma] = pr[ma]; st.ui[fr_row_off(J) + ma] = pi[ma]; }
         fr_col_fwd<T, TJ, J + 1, MB>(st, pr, pi);
@@ -1078,8 +1031,8 @@ __device__ __forceinline__ void fr_add_y(FrState<T, TJ> &st, const typename cplx
 #pragma unroll
     for (int ma = 0; ma <= MAMAX; ma++) {
         const T2 y = yrow[ma * ys];
-        // v-space (FP32): u = unorm v, so the adjoint of the row v is unorm Y
-        const T un = fr_cf<T>() ? unorm<T>(J, MB, ma) : T(1);
+        // u = unorm v, so the adjoint of the row v is unorm Y
+        const T un = unorm<T>(J, MB, ma);
         const T nu = (2 * MB == J && ma == MB) ? T(0.5) * un : un;
         st.lr[ma] += nu * y.x; st.li[ma] += nu * y.y;
     }
@@ -1099,25 +1052,13 @@ __device__ __forceinline__ void fr_col_bwd(FrState<T, TJ> &st, const typename cp
         const T lr = st.lr[ma], li = st.li[ma];
         if (ma < J) {
             const T pr = st.ur[PO + ma], pi = st.ui[PO + ma];
-            if constexpr (fr_cf<T>()) {
-                gar += lr * pr + li * pi;
-                gai += lr * pi - li * pr;
-            } else {
-                const T A = rootpq<T>(J - ma, J - MB);
-                gar += A * (lr * pr + li * pi);
-                gai += A * (lr * pi - li * pr);
-            }
+            gar += lr * pr + li * pi;
+            gai += lr * pi - li * pr;
         }
         if (ma >= 1) {
             const T pr = st.ur[PO + ma - 1], pi = st.ui[PO + ma - 1];
-            if constexpr (fr_cf<T>()) {
-                gbr -= lr * pr + li * pi;
-                gbi -= lr * pi - li * pr;
-            } else {
-                const T B = rootpq<T>(ma, J - MB);
-                gbr -= B * (lr * pr + li * pi);
-                gbi -= B * (lr * pi - li * pr);
-            }
+            gbr -= lr * pr + li * pi;
+            gbi -= lr * pi - li * pr;
         }
     }
     G[0].add(gar); G[1].add(gai); G[2].add(gbr); G[3].add(gbi);
@@ -1125,14 +1066,8 @@ __device__ __forceinline__ void fr_col_bwd(FrState<T, TJ> &st, const typename cp
 #pragma unroll
     for (int k = 0; k < J; k++) {
         const T lr = st.lr[k], li = st.li[k], mr = st.lr[k + 1], mi = st.li[k + 1];
-        if constexpr (fr_cf<T>()) {
-            st.lr[k] = (ar * lr - ai * li) - (br * mr - bi * mi);
-            st.li[k] = (ar * li + ai * lr) - (br * mi + bi * mr);
-        } else {
-            const T A = rootpq<T>(J - k, J - MB), B = rootpq<T>(k + 1, J - MB);
-            st.lr[k] = A * (ar * lr - ai * li) - B * (br * mr - bi * mi);
-            st.li[k] = A * (ar * li + ai * lr) - B * (br * mi + bi * mr);
-        }
+        st.lr[k] = (ar * lr - ai * li) - (br * mr - bi * mi);
+        st.li[k] = (ar * li + ai * lr) - (br * mi + bi * mr);
     }
     if constexpr (J - 1 >= 2 * MB) {
         // parent is row (J-1, MB) of this column
