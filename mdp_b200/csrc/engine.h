@@ -25,6 +25,14 @@ __global__ void k_ghost_count(const double4 *, int, const __grid_constant__ BoxP
 __global__ void k_ghost_emit(double4 *, int *, int, const __grid_constant__ BoxParams, const int *, const unsigned *);
 __global__ void k_cell_index(const double4 *, int, const __grid_constant__ BoxParams, int *, int *);
 __global__ void k_cell_fill(int, const int *, const int *, int *, int *);
+// warps per CTA of k_neigh_build and the ints each keeps for a row of nm slots
+constexpr int NEIGH_WARPS = 4;
+__host__ __device__ inline int neigh_capacity(int nm)
+{
+    int p = 2;
+    while (p < nm) p <<= 1;
+    return p;
+}
 __global__ void k_neigh_build(const double4 *, int, const __grid_constant__ BoxParams, const int *, const int *,
                               const int *, double, int, int *, int *, int *);
 __global__ void k_rev_count(const int *, const int *, const int *, int, int, int *);
@@ -33,8 +41,6 @@ __global__ void k_rev_sort(int, const int *, long long *);
 __global__ void k_pair_count(const double4 *, const int *, const int *, int, int, double, int *);
 __global__ void k_pair_emit(const double4 *, const int *, const int *, int, int, const int *, SnapGeom, double4 *,
                             int2 *, double4 *, int *);
-__global__ void k_tally(const double4 *, const double4 *, const int *, const int *, int, const int *,
-                        const long long *, double4 *, double *, int nblk, int ipad);
 
 // Several element types: type-pair cutoffs (radelem_i + radelem_j) rcutfac,
 // their squares and the neighbour weights wjelem_j (InitSnap,
@@ -164,6 +170,10 @@ int force_compute(ForcePath &fp, const SnapModel &m, int precision, const double
                   const int *nlist, const int *nnum, int nm, long pair_cap, const int *roff,
                   const long long *rlist, double *eatom, double4 *f, double *vatom, cudaStream_t s,
                   const int *atype = nullptr, const int *alist = nullptr);
+
+// forces and virials of inum atoms from the pairs' dE/dr (no atomics)
+void launch_tally(const ForcePath &fp, int inum, const int *roff, const long long *rlist, double4 *f, double *vatom,
+                  int nblk, int ipad, cudaStream_t s);
 
 // Neighbour structure (ghosts + list + reverse list) owned by a caller
 struct Neighbors {

@@ -474,8 +474,7 @@ static int force_compute_me(ForcePath &fp, const SnapModel &m, int precision, co
     if (rc) return rc;
     if (fp.timing) cudaEventRecord(fp.ev[4], s);
     const int gb = (inum + tb - 1) / tb;
-    k_tally<<<gb, tb, 0, s>>>(fp.prij.as<double4>(), fp.dE.as<double4>(), fp.poff.as<int>(), fp.smap.as<int>(), inum,
-                              roff, rlist, f, vatom, nblk, ipad);
+    launch_tally(fp, inum, roff, rlist, f, vatom, nblk, ipad, s);
     count_launches(6);   // elem, pair_count, pair_emit, ui, fi, tally (+ the scan counts itself)
     if (m.zbl.on) {
         k_zbl<<<gb, tb, 0, s>>>(x, nlist, nnum, inum, nm, m.zbl, eatom, f, vatom);
@@ -536,8 +535,7 @@ int force_compute(ForcePath &fp, const SnapModel &m, int precision, const double
     }
     if (rc) return rc;
     if (fp.timing) cudaEventRecord(fp.ev[4], s);
-    k_tally<<<gb, tb, 0, s>>>(fp.prij.as<double4>(), fp.dE.as<double4>(), fp.poff.as<int>(), fp.smap.as<int>(), inum,
-                              roff, rlist, f, vatom, 1, 0);
+    launch_tally(fp, inum, roff, rlist, f, vatom, 1, 0, s);
     count_launches(6);   // pair_count, pair_emit, ui, yi, fi, tally (+ the scan counts itself)
     if (m.zbl.on) {
         k_zbl<<<gb, tb, 0, s>>>(x, nlist, nnum, inum, nm, m.zbl, eatom, f, vatom);
@@ -595,15 +593,17 @@ int neighbor_build(Neighbors &nb, const BoxParams &bp, double4 *x, int inum, dou
     k_cell_fill<<<(anum + tb - 1) / tb, tb, 0, s>>>(anum, nb.cidx.as<int>(), nb.cstart.as<int>(), nb.cursor.as<int>(),
                                                     nb.catoms.as<int>());
     MDP_CUDA_TRY(cudaMemsetAsync(nb.status.p, 0, sizeof(int), s));
-    k_neigh_build<<<(inum + 127) / 128, 128, 0, s>>>(x, inum, bp, nb.cidx.as<int>(), nb.cstart.as<int>(),
+    k_neigh_build<<<(inum + NEIGH_WARPS - 1) / NEIGH_WARPS, NEIGH_WARPS * 32,
+                    sizeof(int) * NEIGH_WARPS * neigh_capacity(nm), s>>>(x, inum, bp, nb.cidx.as<int>(), nb.cstart.as<int>(),
                                                      nb.catoms.as<int>(), rc * rc, nm, nb.nlist.as<int>(),
                                                      nb.nnum.as<int>(), nb.status.as<int>());
     MDP_CUDA_TRY(cudaMemsetAsync(nb.rcount.p, 0, sizeof(int) * inum, s));
-    k_rev_count<<<(inum + tb - 1) / tb, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum,
+    const unsigned gs = (unsigned)(((long)inum * nm + tb - 1) / tb);   // one thread per slot
+    k_rev_count<<<gs, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum,
                                                     nm, nb.rcount.as<int>());
     if (exclusive_scan(nb.rcount.as<int>(), nb.roff.as<int>(), inum, tmp, s)) return -1;
     MDP_CUDA_TRY(cudaMemsetAsync(nb.cursor.p, 0, sizeof(int) * inum, s));
-    k_rev_fill<<<(inum + tb - 1) / tb, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum, nm,
+    k_rev_fill<<<gs, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum, nm,
                                                    nb.roff.as<int>(), nb.cursor.as<int>(), nb.rlist.as<long long>());
     k_rev_sort<<<std::min((inum + 7) / 8, num_sms() * 8), 256, 0, s>>>(inum, nb.roff.as<int>(), nb.rlist.as<long long>());
     count_launches(8);

@@ -662,7 +662,7 @@ int sur_features(Surrogate &S, ForcePath &fp, const double4 *x, int inum, const 
         fp.scan_tmp.ensure(sizeof(int) * scan_tmp_ints(inum)) || S.B.ensure(sizeof(double) * SUR_NK * (size_t)inum) ||
         S.G.ensure(sizeof(float) * SUR_NK * (size_t)inum))
         return -1;
-    const int tb = 256, gb = (inum + tb - 1) / tb;
+    const int tb = 256;
     const unsigned gw = (unsigned)(((long)inum * 32 + tb - 1) / tb);   // one warp per atom
     k_pair_count<<<gw, tb, 0, s>>>(x, nlist, nnum, inum, nm, m.geom.rcutsq, fp.pcount.as<int>());
     if (exclusive_scan(fp.pcount.as<int>(), fp.poff.as<int>(), inum, fp.scan_tmp.as<int>(), s)) return -1;
@@ -687,10 +687,8 @@ int sur_force(Surrogate &S, ForcePath &fp, const double4 *x, int inum, const int
                                                 S.G.as<float>());
     if (launch_yi_pa_f4(S.model, fp, inum, S.G.as<float>(), s)) return -1;
     if (launch_fi<float, 4>(S.model, fp, inum, nm, s)) return -1;
-    const int tb = 256, gb = (inum + tb - 1) / tb;
     if (fp.timing) cudaEventRecord(fp.ev[4], s);
-    k_tally<<<gb, tb, 0, s>>>(fp.prij.as<double4>(), fp.dE.as<double4>(), fp.poff.as<int>(), fp.smap.as<int>(), inum,
-                              roff, rlist, f, vatom, 1, 0);
+    launch_tally(fp, inum, roff, rlist, f, vatom, 1, 0, s);
     count_launches(4);
     if (fp.timing) {
         cudaEventRecord(fp.ev[5], s);

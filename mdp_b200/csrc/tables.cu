@@ -246,6 +246,12 @@ int exclusive_scan(const int *in, int *out, long n, int *tmp, cudaStream_t s)
         MDP_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(int), s));
         return 0;
     }
+    if (nb == 1) {   // one block: its local scan is the whole scan, its sum the total
+        k_scan_local<<<1, SCAN_T, 0, s>>>(in, out, n, out + n);
+        count_launches(1);
+        MDP_CUDA_TRY(cudaGetLastError());
+        return 0;
+    }
     k_scan_local<<<(unsigned)nb, SCAN_T, 0, s>>>(in, out, n, tmp);
     k_scan_top<<<1, SCAN_T, 0, s>>>(tmp, (int)nb, out + n);
     k_scan_add<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, n, tmp);

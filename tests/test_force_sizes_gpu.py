@@ -51,3 +51,25 @@ def test_force_stages_match_oracle(cuda_lib, cells, vac, tj):
     assert rel(out["eatom"], e) < 1e-12 and rel(out["fatom"], f) < 1e-12 and rel(out["vatom"], v) < 1e-12
     out = snap_compute(p, x, box, 1.0, 80, precision="fp32")
     assert rel(out["eatom"], e) < 1e-6 and rel(out["fatom"], f) < 1e-5 and rel(out["vatom"], v) < 1e-5
+
+
+@pytest.mark.parametrize("cells,vac,jitter", [((2, 2, 2), 0, 0.0), ((3, 3, 4), 3, 0.25), ((6, 6, 6), 0, 0.1)])
+def test_neighbour_rows_at_their_capacity(cuda_lib, cells, vac, jitter):
+    """Rows that the fullest atom fills exactly (powers of two and not) equal the
+    oracle's index for index; one slot less is an error."""
+    from mdp_b200 import _lib
+    from mdp_b200.snap import snap_compute
+    p = configs.snap_params(4, seed=11)
+    cfg = configs.ta_config(cells, temp=0.0, jitter=jitter, seed=9)
+    keep = np.ones(cfg.natoms, dtype=bool)
+    keep[:vac] = False
+    x = np.ascontiguousarray(cfg.x[keep])
+    for skin in (0.2, 1.0):
+        xa, al, nl, nn = oracle.neighbor_list(x, cfg.box, p.rcut, skin, 128)
+        nm = int(nn.max())
+        out = snap_compute(p, x, cfg.box, skin, nm, want_neighbors=True)
+        assert np.array_equal(out["neighnum"], nn)
+        for i in range(x.shape[0]):
+            assert np.array_equal(out["neighlist"][i, :nn[i]], np.sort(nl[i, :nn[i]]))
+        with pytest.raises(_lib.MdpError, match="overflow"):
+            snap_compute(p, x, cfg.box, skin, nm - 1)
