@@ -102,6 +102,11 @@ struct mdp_md {
     Neighbors nb;
     ForcePath fp;
     long long step = 0, rebuilds = 0;
+    // rebuild check: the largest squared displacement since the last rebuild, its
+    // pinned copy and the event behind that copy
+    unsigned long long *hmax = nullptr;
+    cudaEvent_t emax = nullptr;
+    double disp_last = 0.0;
     double thermo_last[5] = {0, 0, 0, 0, 0};
     bool ready = false;
     // learned surrogate: driving model, judge cadence and tolerance, fallback
@@ -150,6 +155,8 @@ int mdp_md_create(mdp_md **h, const mdp_snap_params *p, const mdp_md_config *cfg
     m->anum_cap = (long)ceil(1.3 * vol * cfg->natoms) + 1024;
     const long n = cfg->natoms;
     if (cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMallocHost((void **)&m->hmax, sizeof(*m->hmax)) != cudaSuccess ||
+        cudaEventCreateWithFlags(&m->emax, cudaEventDisableTiming) != cudaSuccess ||
         m->x.ensure(sizeof(double4) * m->anum_cap) || m->v.ensure(sizeof(double4) * n) ||
         m->f.ensure(sizeof(double4) * n) || m->xstart.ensure(sizeof(double4) * n) ||
         m->xhold.ensure(sizeof(double4) * n) || m->e.ensure(sizeof(double) * n) ||
@@ -171,6 +178,8 @@ void mdp_md_destroy(mdp_md *m)
     for (auto x : b) x->release();
     m->nb.release();
     m->fp.release();
+    if (m->emax) cudaEventDestroy(m->emax);
+    if (m->hmax) cudaFreeHost(m->hmax);
     if (m->s) cudaStreamDestroy(m->s);
     delete m;
 }
@@ -215,6 +224,7 @@ static int md_rebuild(mdp_md *m)
     const double rc = m->model.geom.rcut + m->cfg.skin;
     if (neighbor_build(m->nb, m->bp, m->x.as<double4>(), n, rc, m->cfg.neighmax, m->anum_cap, m->s)) return -1;
     MDP_CUDA_TRY(cudaMemcpyAsync(m->xhold.p, m->x.p, sizeof(double4) * n, cudaMemcpyDeviceToDevice, m->s));
+    m->disp_last = 0.0;
     m->rebuilds++;
     return 0;
 }
@@ -228,6 +238,23 @@ static int md_force_plain(mdp_md *m)
                          m->s, m->has_types ? m->types.as<int>() : nullptr, m->nb.alist.as<int>());
 }
 
+// ghosts follow their owners' displacement of this step
+static int md_shift(mdp_md *m)
+{
+    if (m->nb.gnum > 0) {
+        k_ghost_shift<<<(m->nb.gnum + 255) / 256, 256, 0, m->s>>>(m->x.as<double4>(), m->xstart.as<double4>(),
+                                                                  m->nb.alist.as<int>(), m->cfg.natoms, m->nb.gnum);
+        count_launches(1);
+    }
+    return 0;
+}
+
+// the force of this step is judged: it reads results back on the host
+static bool md_judged(const mdp_md *m)
+{
+    return m->sur && m->fallback_step < 0 && m->judge_every > 0 && m->step % m->judge_every == 0;
+}
+
 // Surrogate forces, judged against the plain model every judge_every steps:
 // the plain forces replace the surrogate's on a judged step, and a force RMSE
 // above the tolerance hands the run to the plain model from then on.
@@ -239,7 +266,7 @@ static int md_force(mdp_md *m)
                   m->cfg.neighmax, m->nb.roff.as<int>(), m->nb.rlist.as<long long>(), m->e.as<double>(),
                   m->f.as<double4>(), m->vatom.as<double>(), m->s))
         return -1;
-    if (m->judge_every <= 0 || m->step % m->judge_every != 0) return 0;
+    if (!md_judged(m)) return 0;
     if (m->fjudge.ensure(sizeof(double4) * (size_t)n)) return -1;
     MDP_CUDA_TRY(cudaMemcpyAsync(m->fjudge.p, m->f.p, sizeof(double4) * (size_t)n, cudaMemcpyDeviceToDevice, m->s));
     if (md_force_plain(m)) return -1;
@@ -317,7 +344,7 @@ int mdp_md_run(mdp_md *m, int nsteps, int thermo_every, double *thermo, int ther
     const double dtf = 0.5 * m->cfg.dt * FTM2V;   // readdata.cpp:418-420
     const double dtfm = dtf / m->cfg.mass;
     const double dtv = m->cfg.dt;
-    const double skin = m->cfg.skin;
+    const double limit = 0.25 * m->cfg.skin * m->cfg.skin;   // rebuild when an atom has moved more than skin / 2
     int rows = 0;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -330,29 +357,34 @@ int mdp_md_run(mdp_md *m, int nsteps, int thermo_every, double *thermo, int ther
                                                          m->xstart.as<double4>(), n, dtfm, dtv);
         count_launches(1);
         const long long ago = m->step;
-        int build = 0;
+        int build = 0, ahead = 0;
         if (ago >= m->cfg.neighdelay && ago % m->cfg.neighevery == 0) {
             if (!m->cfg.neighcheck) build = 1;
             else {
                 MDP_CUDA_TRY(cudaMemsetAsync(dmax, 0, sizeof(unsigned long long), m->s));
                 k_maxdisp<<<(n + 255) / 256, 256, 0, m->s>>>(m->x.as<double4>(), m->xhold.as<double4>(), n, dmax);
                 count_launches(1);
-                unsigned long long hm = 0;
-                MDP_CUDA_TRY(cudaMemcpyAsync(&hm, dmax, sizeof(hm), cudaMemcpyDeviceToHost, m->s));
-                MDP_CUDA_TRY(cudaStreamSynchronize(m->s));
+                MDP_CUDA_TRY(cudaMemcpyAsync(m->hmax, dmax, sizeof(unsigned long long), cudaMemcpyDeviceToHost, m->s));
+                MDP_CUDA_TRY(cudaEventRecord(m->emax, m->s));
+                // Queue the force on the kept list before waiting for the check,
+                // while the last one was well inside the limit: the GPU works on
+                // through the wait (128 atoms: the host's round trip is a tenth of
+                // a step).  Should a rebuild be due after all, its own force
+                // evaluation overwrites this one's results.
+                ahead = m->disp_last < 0.81 * limit && !m->fp.timing && !md_judged(m);
+                if (ahead && (md_shift(m) || md_force(m))) return -1;
+                MDP_CUDA_TRY(cudaEventSynchronize(m->emax));
                 double md;
-                memcpy(&md, &hm, sizeof(md));
-                if (md > 0.25 * skin * skin) build = 1;
+                memcpy(&md, m->hmax, sizeof(md));
+                m->disp_last = md;
+                if (md > limit) build = 1;
             }
         }
         if (build) {
-            if (md_rebuild(m)) return -1;
-        } else if (m->nb.gnum > 0) {
-            k_ghost_shift<<<(m->nb.gnum + 255) / 256, 256, 0, m->s>>>(m->x.as<double4>(), m->xstart.as<double4>(),
-                                                                      m->nb.alist.as<int>(), n, m->nb.gnum);
-            count_launches(1);
+            if (md_rebuild(m) || md_force(m)) return -1;
+        } else if (!ahead) {
+            if (md_shift(m) || md_force(m)) return -1;
         }
-        if (md_force(m)) return -1;
         k_nve_final<<<(n + 255) / 256, 256, 0, m->s>>>(m->v.as<double4>(), m->f.as<double4>(), n, dtfm);
         count_launches(1);
         if (thermo_every > 0 && m->step % thermo_every == 0) {
