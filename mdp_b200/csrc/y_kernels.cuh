@@ -14,6 +14,7 @@
 
 #include "engine.h"
 
+#include <algorithm>
 #include <array>
 
 
@@ -28,6 +29,8 @@ template <int TJ> __host__ __device__ constexpr int yj_top(int r)
     const int q = r - TJ - 1;
     return (q & 1) ? q : -(q + 1);
 }
+// a top that no coupling reaches (a warp without a job keeps the others' step)
+template <int TJ> __host__ __device__ constexpr int yj_none(int par) { return -2 * TJ - 2 - par; }
 // accumulators: left half columns ma <= J/2 of the layers of one parity
 __host__ __device__ constexpr int yacc_off(int J)
 {
@@ -46,9 +49,9 @@ template <int TJ> __host__ __device__ constexpr int yacc_count(int par)
 // holds) is fetched about once per parity and CTA.  Instruction fetch is what
 // bounds this kernel: the same jobs one after the other on fewer warps took
 // 32.5 ns per atom at 250,000 atoms (FP64, 2J = 8) when the warps shared every
-// job and 196 ns when each warp worked on a job of its own, against 18.0 ns in
-// this form.  A barrier per coupling, to keep the warps in step, costs more
-// than it saves (18.6 ns).  FP32 needs half the registers, so two tiles share
+// job and 196 ns when each warp worked on a job of its own, against 16.2 ns in
+// this form.  A barrier after each J1 keeps the warps in step (FP64 16.2 ns, FP32
+// 8.7; without 18.0 and 9.0; one per coupling 18.6 and 9.8).  FP32 needs half the registers, so two tiles share
 // a CTA and the fetched code.
 template <int TJ> __host__ __device__ constexpr int y_warps() { return TJ >= 6 ? 12 : 8; }
 template <typename T, int TJ> __host__ __device__ constexpr int y_tiles() { return sizeof(T) == 4 && TJ == 8 ? 2 : 1; }
@@ -56,7 +59,7 @@ template <typename T, int TJ> __host__ __device__ constexpr int y_tiles() { retu
 // Per parity and warp: the job (255: none) and which of every `st` items of it
 // the warp takes, starting with the o-th; the warps of a job shared by two meet
 // in shared-memory zone `zone`.  block[g][parity]: the couplings of group g.
-constexpr int Y_MAXG = 8, Y_MAXW = 12, Y_ZONES = 6;
+constexpr int Y_MAXG = 8, Y_MAXW = 12;
 struct YPlan {
     unsigned char job[2][Y_MAXW], o[2][Y_MAXW], st[2][Y_MAXW], zone[2][Y_MAXW];
     unsigned block[Y_MAXG][2];
@@ -112,27 +115,48 @@ __device__ __forceinline__ void y_products(T (&tr)[YC<TJ, J1, J2>::nj], T (&ti)[
         y_products<T, TJ, J1, J2, M, A + 1, Q0>(tr, ti, ar, ai, br, bi);
     }
 }
-template <typename T, int TJ, int J1, int J2, int M, int Q>
-__device__ __forceinline__ void y_store(T (&yr)[yacc_count<TJ>((J1 + J2) & 1)],
-                                        T (&yi)[yacc_count<TJ>((J1 + J2) & 1)], const T (&tr)[YC<TJ, J1, J2>::nj],
+// sums of one job: the Y entries, and with EN the part of them that is the
+// energy's derivative by U_J alone (see k_snap_y_me)
+template <typename T, int N, bool EN = false> struct YSums {
+    T r[N], i[N], er[EN ? N : 1], ei[EN ? N : 1];
+    __device__ __forceinline__ void zero()
+    {
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            r[k] = T(0); i[k] = T(0);
+            if constexpr (EN) { er[k] = T(0); ei[k] = T(0); }
+        }
+    }
+    // layer J of coupling (J1, J2): s t added to accumulator K
+    template <int J1, int J2, int J, int K> __device__ __forceinline__ void add(const T s, const T tr, const T ti)
+    {
+        r[K] += s * tr;
+        i[K] += s * ti;
+        if constexpr (EN && J >= J1) {
+            constexpr double w = J == J1 ? (J2 == J ? 1.0 / 3.0 : 0.5) : 1.0;   // without the multiplicity
+            er[K] += T(w) * s * tr;
+            ei[K] += T(w) * s * ti;
+        }
+    }
+};
+template <typename T, int TJ, int J1, int J2, int M, int Q, typename Out>
+__device__ __forceinline__ void y_store(Out &out, const T (&tr)[YC<TJ, J1, J2>::nj],
                                         const T (&ti)[YC<TJ, J1, J2>::nj], const T (&sj)[YC<TJ, J1, J2>::nj])
 {
     typedef YC<TJ, J1, J2> C;
     if constexpr (Q < C::nj) {
         constexpr int J = C::jlo + 2 * Q, K = yacc_off(J) + M - (J1 + J2 - J) / 2;
-        yr[K] += sj[Q] * tr[Q];
-        yi[K] += sj[Q] * ti[Q];
-        y_store<T, TJ, J1, J2, M, Q + 1>(yr, yi, tr, ti, sj);
+        out.template add<J1, J2, J, K>(sj[Q], tr[Q], ti[Q]);
+        y_store<T, TJ, J1, J2, M, Q + 1>(out, tr, ti, sj);
     }
 }
 // columns ma1 + ma2 = M.. of one row pair; the centre column (even layers,
 // m = 0) belongs to the jobs with m' <= 0
-template <typename T, int TJ, int J1, int J2, int M>
-__device__ __forceinline__ void y_columns(T (&yr)[yacc_count<TJ>((J1 + J2) & 1)],
-                                          T (&yi)[yacc_count<TJ>((J1 + J2) & 1)],
-                                          const T (&ar)[YC<TJ, J1, J2>::n1], const T (&ai)[YC<TJ, J1, J2>::n1],
-                                          const T (&br)[YC<TJ, J1, J2>::n2], const T (&bi)[YC<TJ, J1, J2>::n2],
-                                          const T (&sj)[YC<TJ, J1, J2>::nj], const int top)
+template <typename T, int TJ, int J1, int J2, int M, typename Out>
+__device__ __forceinline__ void y_columns(Out &out, const T (&ar)[YC<TJ, J1, J2>::n1],
+                                          const T (&ai)[YC<TJ, J1, J2>::n1], const T (&br)[YC<TJ, J1, J2>::n2],
+                                          const T (&bi)[YC<TJ, J1, J2>::n2], const T (&sj)[YC<TJ, J1, J2>::nj],
+                                          const int top)
 {
     typedef YC<TJ, J1, J2> C;
     if constexpr (M <= C::mc) {
@@ -142,50 +166,60 @@ __device__ __forceinline__ void y_columns(T (&yr)[yacc_count<TJ>((J1 + J2) & 1)]
             if (AM > 0 || top <= 0) {
                 T tr[C::nj], ti[C::nj];
                 y_products<T, TJ, J1, J2, M, cmax(0, M - J2), Q0>(tr, ti, ar, ai, br, bi);
-                y_store<T, TJ, J1, J2, M, Q0>(yr, yi, tr, ti, sj);
+                y_store<T, TJ, J1, J2, M, Q0>(out, tr, ti, sj);
             }
         }
-        y_columns<T, TJ, J1, J2, M + 1>(yr, yi, ar, ai, br, bi, sj, top);
+        y_columns<T, TJ, J1, J2, M + 1>(out, ar, ai, br, bi, sj, top);
     }
 }
-template <typename T, int TJ, bool PA, int J1, int J2, int Q>
-__device__ __forceinline__ void y_scale(T (&sj)[YC<TJ, J1, J2>::nj], const int mb1, const int mb2,
-                                        const YParams<T> &P, const T *__restrict__ Gs)
+// coefficient of coupling (J1, J2, J): the model's, or times the atom's own (PA)
+template <typename T, bool PA> struct YScale {
+    const YParams<T> &P;
+    const T *Gs;
+    template <int J1, int J2, int J> __device__ __forceinline__ T get() const
+    {
+        constexpr int TRI = tri_index(J1, J2, J);
+        T b = P.betaY[TRI];
+        if constexpr (PA) b *= Gs[P.kmap[TRI] * 32];
+        return b;
+    }
+};
+template <typename T, int TJ, int J1, int J2, int Q, typename Scale>
+__device__ __forceinline__ void y_scale(T (&sj)[YC<TJ, J1, J2>::nj], const int mb1, const int mb2, const Scale &sc,
+                                        const bool sym)
 {
     typedef YC<TJ, J1, J2> C;
     if constexpr (Q < C::nj) {
-        constexpr int J = C::jlo + 2 * Q, TRI = tri_index(J1, J2, J), CGB = cg_block(J1, J2, J);
-        T b = P.betaY[TRI];
-        if constexpr (PA) b *= Gs[P.kmap[TRI] * 32];
-        sj[Q] = b * cgc<T>(CGB + mb1 * (J2 + 1) + mb2);
-        if (J1 == J2 && mb1 != mb2) sj[Q] += sj[Q];
-        y_scale<T, TJ, PA, J1, J2, Q + 1>(sj, mb1, mb2, P, Gs);
+        constexpr int J = C::jlo + 2 * Q, CGB = cg_block(J1, J2, J);
+        sj[Q] = sc.template get<J1, J2, J>() * cgc<T>(CGB + mb1 * (J2 + 1) + mb2);
+        if (J1 == J2 && sym && mb1 != mb2) sj[Q] += sj[Q];
+        y_scale<T, TJ, J1, J2, Q + 1>(sj, mb1, mb2, sc, sym);
     }
 }
 
-// the warp's share of one coupling pair (J1, J2) of a job.  J1 = J2: exchanging
-// the factors gives the same term, so only mb1 <= mb2 is walked (twice the
-// weight off the diagonal).
-template <typename T, int TJ, bool PA, int J1, int J2>
-__device__ __forceinline__ void y_block(T (&yr)[yacc_count<TJ>((J1 + J2) & 1)],
-                                        T (&yi)[yacc_count<TJ>((J1 + J2) & 1)],
-                                        const typename cplx<T>::type *__restrict__ Us, const int top,
-                                        const YParams<T> &P, const T *__restrict__ Gs, int &next, const int st)
+// the warp's share of one coupling pair (J1, J2) of a job, the J1 factor from
+// U1, the J2 factor from U2.  J1 = J2 and the same U (sym): exchanging the
+// factors gives the same term, so only mb1 <= mb2 is walked (twice the weight
+// off the diagonal).
+template <typename T, int TJ, int J1, int J2, typename Scale, typename Out>
+__device__ __forceinline__ void y_block(Out &out, const typename cplx<T>::type *__restrict__ U1,
+                                        const typename cplx<T>::type *__restrict__ U2, const int top,
+                                        const Scale &sc, const bool sym, int &next, const int st)
 {
     typedef YC<TJ, J1, J2> C;
     if constexpr (C::nj > 0) {
         const int s = (top + J1 + J2) >> 1;   // mb1 + mb2
         if (s < 0 || s > J1 + J2) return;
-        const int hi = J1 == J2 ? (s >> 1) : min(J1, s);
+        const int hi = J1 == J2 && sym ? (s >> 1) : min(J1, s);
         int mb1 = max(0, s - J2) + next;
 #pragma unroll 1
         for (; mb1 <= hi; mb1 += st) {
             const int mb2 = s - mb1;
             T ar[C::n1], ai[C::n1], br[C::n2], bi[C::n2], sj[C::nj];
-            y_load_row<T, J1, C::n1>(Us, mb1, ar, ai);
-            y_load_row<T, J2, C::n2>(Us, mb2, br, bi);
-            y_scale<T, TJ, PA, J1, J2, 0>(sj, mb1, mb2, P, Gs);
-            y_columns<T, TJ, J1, J2, 0>(yr, yi, ar, ai, br, bi, sj, top);
+            y_load_row<T, J1, C::n1>(U1, mb1, ar, ai);
+            y_load_row<T, J2, C::n2>(U2, mb2, br, bi);
+            y_scale<T, TJ, J1, J2, 0>(sj, mb1, mb2, sc, sym);
+            y_columns<T, TJ, J1, J2, 0>(out, ar, ai, br, bi, sj, top);
         }
         next = mb1 - hi - 1;
     }
@@ -201,28 +235,31 @@ __host__ __device__ constexpr int y_bit(int j1, int j2)
     return n;
 }
 
-template <typename T, int TJ, bool PA, int PAR, int J1, int J2>
-__device__ __forceinline__ void y_couplings(T (&yr)[yacc_count<TJ>(PAR)], T (&yi)[yacc_count<TJ>(PAR)],
-                                            const typename cplx<T>::type *__restrict__ Us, const int top,
-                                            const YParams<T> &P, const T *__restrict__ Gs, int &next, const int st,
+// All couplings of a parity, with a barrier after each J1 that keeps the CTA's
+// warps in step (every warp calls this the same number of times).
+template <typename T, int TJ, int PAR, int J1, int J2, typename Scale, typename Out>
+__device__ __forceinline__ void y_couplings(Out &out, const typename cplx<T>::type *__restrict__ U1,
+                                            const typename cplx<T>::type *__restrict__ U2, const int top,
+                                            const Scale &sc, const bool sym, int &next, const int st,
                                             const unsigned blocks)
 {
     if constexpr (J1 <= TJ) {
         if constexpr (J2 <= J1) {
             if constexpr (((J1 + J2) & 1) == PAR) {
-                if (blocks >> y_bit(J1, J2) & 1) y_block<T, TJ, PA, J1, J2>(yr, yi, Us, top, P, Gs, next, st);
+                if (blocks >> y_bit(J1, J2) & 1) y_block<T, TJ, J1, J2>(out, U1, U2, top, sc, sym, next, st);
             }
-            y_couplings<T, TJ, PA, PAR, J1, J2 + 1>(yr, yi, Us, top, P, Gs, next, st, blocks);
+            y_couplings<T, TJ, PAR, J1, J2 + 1>(out, U1, U2, top, sc, sym, next, st, blocks);
         } else {
-            y_couplings<T, TJ, PA, PAR, J1 + 1, 0>(yr, yi, Us, top, P, Gs, next, st, blocks);
+            if constexpr (J1 >= 3) __syncthreads();
+            y_couplings<T, TJ, PAR, J1 + 1, 0>(out, U1, U2, top, sc, sym, next, st, blocks);
         }
     }
 }
 
-// a finished job's outputs to Y (half plane), its energy share into e
-template <typename T, int TJ, bool PA, int J>
-__device__ __forceinline__ void y_finish(T (&yr)[yacc_count<TJ>(J & 1)], T (&yi)[yacc_count<TJ>(J & 1)],
-                                         const typename cplx<T>::type *__restrict__ Us,
+// a finished job's outputs to Y (half plane); with EN != 0 its energy share into
+// e: sum w Re(U* Y) (EN 1), or of the energy's own sums (EN 2)
+template <typename T, int TJ, int EN, int J, typename Sums>
+__device__ __forceinline__ void y_finish(const Sums &a, const typename cplx<T>::type *__restrict__ Us,
                                          typename cplx<T>::type *__restrict__ dst, const int top, double &e)
 {
     typedef typename cplx<T>::type T2;
@@ -237,59 +274,65 @@ __device__ __forceinline__ void y_finish(T (&yr)[yacc_count<TJ>(J & 1)], T (&yi)
 #pragma unroll
             for (int ma = 0; 2 * ma <= J; ma++) {
                 if (2 * ma == J && mir) continue;
-                T2 y = T2{yr[yacc_off(J) + ma], yi[yacc_off(J) + ma]};
-                if (mir) {
-                    if ((ma + mb) & 1) y.x = -y.x; else y.y = -y.y;
-                }
+                constexpr int O = yacc_off(J);
+                const bool nx = mir && ((ma + mb) & 1), ny = mir && !nx;   // signs of the mirror image
+                const T2 y = T2{nx ? -a.r[O + ma] : a.r[O + ma], ny ? -a.i[O + ma] : a.i[O + ma]};
                 row[ma * st] = y;
-                if constexpr (!PA) {
+                if constexpr (EN != 0) {
                     const double wgt = (top == 0 && 2 * ma == J) ? 0.5 : 1.0;
                     const T2 u = us[ma * st];
-                    e += wgt * ((double)u.x * (double)y.x + (double)u.y * (double)y.y);
+                    T2 w = y;
+                    if constexpr (EN == 2) w = T2{nx ? -a.er[O + ma] : a.er[O + ma], ny ? -a.ei[O + ma] : a.ei[O + ma]};
+                    e += wgt * ((double)u.x * (double)w.x + (double)u.y * (double)w.y);
                 }
             }
         }
-        y_finish<T, TJ, PA, J - 2>(yr, yi, Us, dst, top, e);
+        y_finish<T, TJ, EN, J - 2>(a, Us, dst, top, e);
     }
 }
 
-// the warp's job of one parity
+// shared-memory zones of the jobs two warps share, per parity, and their offset
+template <int TJ> __host__ __device__ constexpr int y_zones(int par) { return y_warps<TJ>() - (par ? TJ : TJ + 1); }
+template <int TJ> __host__ __device__ constexpr int y_zone_off(int par, int zone)
+{
+    return par ? y_zones<TJ>(0) * yacc_count<TJ>(0) + zone * yacc_count<TJ>(1) : zone * yacc_count<TJ>(0);
+}
+
+// the warp's job of one parity; the warps of a shared job meet in its zone
 template <typename T, int TJ, bool PA, int PAR>
 __device__ __forceinline__ void y_job(const YPlan &plan, const unsigned blocks,
                                       const typename cplx<T>::type *__restrict__ Us,
                                       typename cplx<T>::type *__restrict__ red,
-                                      typename cplx<T>::type *__restrict__ dst, const int w, const YParams<T> &P,
-                                      const T *__restrict__ Gs, double &e)
+                                      typename cplx<T>::type *__restrict__ dst, const int w,
+                                      const YScale<T, PA> &sc, double &e)
 {
     typedef typename cplx<T>::type T2;
     constexpr int NA = yacc_count<TJ>(PAR);
     const int job = plan.job[PAR][w], o = plan.o[PAR][w], st = plan.st[PAR][w];
-    const int top = job == 255 ? -2 * TJ - 2 - PAR : yj_top<TJ>(job);   // none: no coupling reaches it
-    T yr[NA], yi[NA];
-#pragma unroll
-    for (int k = 0; k < NA; k++) { yr[k] = T(0); yi[k] = T(0); }
+    const int top = job == 255 ? yj_none<TJ>(PAR) : yj_top<TJ>(job);
+    YSums<T, NA> a;
+    a.zero();
     int next = o;
-    y_couplings<T, TJ, PA, PAR, 0, 0>(yr, yi, Us, top, P, Gs, next, st, blocks);
-    T2 *z = red + plan.zone[PAR][w] * yacc_count<TJ>(0) * 32;
-    __syncthreads();   // the other parity's zones have been read
+    y_couplings<T, TJ, PAR, 0, 0>(a, Us, Us, top, sc, true, next, st, blocks);
+    T2 *z = red + y_zone_off<TJ>(PAR, plan.zone[PAR][w]) * 32;
     if (o == 1)
 #pragma unroll
-        for (int k = 0; k < NA; k++) z[k * 32] = T2{yr[k], yi[k]};
+        for (int k = 0; k < NA; k++) z[k * 32] = T2{a.r[k], a.i[k]};
     __syncthreads();
     if (job == 255 || o == 1) return;
     if (st == 2)
 #pragma unroll
         for (int k = 0; k < NA; k++) {
             const T2 v = z[k * 32];
-            yr[k] += v.x;
-            yi[k] += v.y;
+            a.r[k] += v.x;
+            a.i[k] += v.y;
         }
-    y_finish<T, TJ, PA, TJ - PAR>(yr, yi, Us, dst, top, e);
+    y_finish<T, TJ, PA ? 0 : 1, TJ - PAR>(a, Us, dst, top, e);
 }
 
 template <typename T, int TJ, bool PA> constexpr size_t y_smem_bytes()
 {
-    return y_tiles<T, TJ>() * (((size_t)idxu_count(TJ) + Y_ZONES * yacc_count<TJ>(0)) * 32 * sizeof(typename cplx<T>::type) +
+    return y_tiles<T, TJ>() * (((size_t)idxu_count(TJ) + y_zone_off<TJ>(1, y_zones<TJ>(1))) * 32 * sizeof(typename cplx<T>::type) +
                                (PA ? (size_t)nbispec(TJ) * 32 * sizeof(T) : (size_t)y_warps<TJ>() * 32 * sizeof(double)));
 }
 
@@ -299,16 +342,16 @@ template <typename T, int TJ, bool PA> constexpr size_t y_smem_bytes()
 // group: eatom is written.  Several groups share the couplings of every tile (few
 // tiles): group g writes its partial Y to Y + g * gstride and its energy share
 // to esum[g * natoms + atom], and k_y_sum adds them up.  PA: per-atom coefficients
-// G[k * natoms + atom] in place of the model's, no energy.
+// G[k * gpitch + atom] in place of the model's, no energy.
 template <typename T, int TJ, bool PA>
 __global__ void __launch_bounds__(y_tiles<T, TJ>() * y_warps<TJ>() * 32, 1)
 k_snap_y(const typename cplx<T>::type *__restrict__ Ut, int natoms, const __grid_constant__ YParams<T> P,
          const __grid_constant__ YPlan plan, int ngroups, typename cplx<T>::type *__restrict__ Y, size_t gstride,
-         double *__restrict__ eatom, double *__restrict__ esum, const T *__restrict__ G)
+         double *__restrict__ eatom, double *__restrict__ esum, const T *__restrict__ G, int gpitch)
 {
     typedef typename cplx<T>::type T2;
     constexpr int NW = y_warps<TJ>(), NT = NW * 32, NTI = y_tiles<T, TJ>();
-    constexpr int NU = idxu_count(TJ), NZ = Y_ZONES * yacc_count<TJ>(0);
+    constexpr int NU = idxu_count(TJ), NZ = y_zone_off<TJ>(1, y_zones<TJ>(1));
     extern __shared__ __align__(16) unsigned char smraw[];
     const int lane = threadIdx.x & 31, sub = threadIdx.x / NT, t = threadIdx.x - sub * NT, w = t >> 5;
     T2 *Us = reinterpret_cast<T2 *>(smraw) + sub * (NU + NZ) * 32;
@@ -324,15 +367,16 @@ k_snap_y(const typename cplx<T>::type *__restrict__ Ut, int natoms, const __grid
     if constexpr (PA) {
         for (int k = t; k < nbispec(TJ) * 32; k += NT) {
             const int a = tile * 32 + (k & 31);
-            Gs[k] = (a < natoms) ? G[(size_t)(k >> 5) * natoms + a] : T(0);
+            Gs[k] = (a < natoms) ? G[(size_t)(k >> 5) * gpitch + a] : T(0);
         }
     }
     __syncthreads();
     double e = 0.0;
     // a missing tile's results go where no one reads them: its own shared tile
     T2 *dst = on ? Y + g * gstride + (size_t)tile * yh_count(TJ) * 32 + lane : Us + lane;
-    y_job<T, TJ, PA, 0>(plan, plan.block[g][0], Us + lane, red + lane, dst, w, P, Gs + lane, e);
-    y_job<T, TJ, PA, 1>(plan, plan.block[g][1], Us + lane, red + lane, dst, w, P, Gs + lane, e);
+    const YScale<T, PA> sc{P, Gs + lane};
+    y_job<T, TJ, PA, 0>(plan, plan.block[g][0], Us + lane, red + lane, dst, w, sc, e);
+    y_job<T, TJ, PA, 1>(plan, plan.block[g][1], Us + lane, red + lane, dst, w, sc, e);
     if constexpr (!PA) {
         ered[w * 32 + lane] = e;
         __syncthreads();
@@ -406,8 +450,7 @@ template <int TJ> void y_plan(YPlan &pl, int ngroups)
                 nb++;
             }
         // spare warps join the heaviest jobs
-        int zones = 0;
-        for (int spare = NW - nj; spare > 0 && zones < Y_ZONES; spare--, zones++) {
+        for (int spare = NW - nj; spare > 0; spare--) {
             int best = -1;
             for (int r = 0; r < nj; r++)
                 if (st[r] == 1 && (best < 0 || cost[r] > cost[best])) best = r;
@@ -458,49 +501,69 @@ template <int TJ> void y_plan(YPlan &pl, int ngroups)
     }
 }
 
-// Groups: as many as keep every CTA in the first wave.  Splitting a tile's
-// couplings over CTAs shortens the stream of instructions each has to fetch
-// (FP64, 2J = 8: 128 atoms 75 us in one group, 31 us in eight; 2,000 atoms 96
-// us in one, 54 us in two, 66 us in four, which needs two waves); with more
+// Groups of ctas CTAs: as many as keep every CTA in one wave.  Splitting a
+// tile's couplings over CTAs shortens the stream of instructions each has to
+// fetch (FP64, 2J = 8: 128 atoms 75 us in one group, 31 us in eight; 2,000 atoms
+// 96 us in one, 54 us in two, 66 us in four, which needs two waves); with more
 // tiles than half the SMs it only adds partial results to sum.  At 2J = 4 the
 // code is short and one group is the fastest at every size.
-template <typename T, int TJ> int y_groups(int ntiles, int sms)
+template <int TJ> int y_groups(int ctas, int wave)
 {
     if (TJ <= 4) return 1;
-    const int ctas = (ntiles + y_tiles<T, TJ>() - 1) / y_tiles<T, TJ>(), g = sms / ctas;
+    const int g = wave / ctas;
     return g < 1 ? 1 : g > Y_MAXG ? Y_MAXG : g;
 }
 
-// Y (and, without G, the energies) of inum atoms from fp.Ut into fp.Y
+// Y (and, without G, the energies) of the atoms from tile t0 on, nt tiles
 template <typename T, int TJ, bool PA>
-int launch_y(const YParams<T> &yp, ForcePath &fp, int inum, double *eatom, const T *G, cudaStream_t s)
+int launch_y_part(const YParams<T> &yp, ForcePath &fp, int inum, int t0, int nt, int wave, double *eatom, const T *G,
+                  cudaStream_t s)
 {
     typedef typename cplx<T>::type T2;
-    if (tu_ensure_tables()) return -1;
-    constexpr int NT = y_tiles<T, TJ>() * y_warps<TJ>() * 32;
+    constexpr int NTI = y_tiles<T, TJ>(), NT = NTI * y_warps<TJ>() * 32;
     const size_t sm = y_smem_bytes<T, TJ, PA>();
-    int per_sm = 0;
-    if (kernel_setup((const void *)k_snap_y<T, TJ, PA>, NT, sm, &per_sm, "k_snap_y")) return -1;
     static const std::array<YPlan, Y_MAXG> plans = [] {
         std::array<YPlan, Y_MAXG> p;
         for (int g = 0; g < Y_MAXG; g++) y_plan<TJ>(p[g], g + 1);
         return p;
     }();
-    const int ntiles = (inum + 31) / 32, ctas = (ntiles + y_tiles<T, TJ>() - 1) / y_tiles<T, TJ>();
-    const int ng = y_groups<T, TJ>(ntiles, num_sms());
-    const size_t n = (size_t)ntiles * yh_count(TJ) * 32;
+    const int atoms = std::min(nt * 32, inum - t0 * 32), ctas = (nt + NTI - 1) / NTI, ng = y_groups<TJ>(ctas, wave);
+    const size_t n = (size_t)nt * yh_count(TJ) * 32;
+    const T2 *U = fp.Ut.as<T2>() + (size_t)t0 * idxu_count(TJ) * 32;
+    T2 *Y = fp.Y.as<T2>() + (size_t)t0 * yh_count(TJ) * 32;
+    if (eatom) eatom += t0 * 32;
+    if (G) G += t0 * 32;
     if (ng == 1) {
-        k_snap_y<T, TJ, PA><<<ctas, NT, sm, s>>>(fp.Ut.as<T2>(), inum, yp, plans[0], 1, fp.Y.as<T2>(), n, eatom,
-                                                  nullptr, G);
+        k_snap_y<T, TJ, PA><<<ctas, NT, sm, s>>>(U, atoms, yp, plans[0], 1, Y, n, eatom, nullptr, G, inum);
         return 0;
     }
-    if (fp.Ypart.ensure(sizeof(T2) * n * ng) || fp.esum.ensure(sizeof(double) * (size_t)inum * ng)) return -1;
-    k_snap_y<T, TJ, PA><<<ctas * ng, NT, sm, s>>>(fp.Ut.as<T2>(), inum, yp, plans[ng - 1], ng, fp.Ypart.as<T2>(), n,
-                                                   eatom, fp.esum.as<double>(), G);
-    k_y_sum<T2><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(fp.Ypart.as<T2>(), n, ng, fp.Y.as<T2>(),
-                                                            fp.esum.as<double>(), inum, yp.e0, PA ? nullptr : eatom);
+    if (fp.Ypart.ensure(sizeof(T2) * n * ng) || fp.esum.ensure(sizeof(double) * (size_t)atoms * ng)) return -1;
+    k_snap_y<T, TJ, PA><<<ctas * ng, NT, sm, s>>>(U, atoms, yp, plans[ng - 1], ng, fp.Ypart.as<T2>(), n, eatom,
+                                                   fp.esum.as<double>(), G, inum);
+    k_y_sum<T2><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(fp.Ypart.as<T2>(), n, ng, Y, fp.esum.as<double>(), atoms,
+                                                            yp.e0, PA ? nullptr : eatom);
     count_launches(1);
     return 0;
+}
+
+// All tiles.  A last wave that is at most half full, after a few full ones, runs
+// by itself with its couplings shared (a wave of one group takes 96 us at
+// 2J = 8, one of two groups 54).
+template <typename T, int TJ, bool PA>
+int launch_y(const YParams<T> &yp, ForcePath &fp, int inum, double *eatom, const T *G, cudaStream_t s)
+{
+    if (tu_ensure_tables()) return -1;
+    constexpr int NTI = y_tiles<T, TJ>(), NT = NTI * y_warps<TJ>() * 32;
+    int per_sm = 0;
+    if (kernel_setup((const void *)k_snap_y<T, TJ, PA>, NT, y_smem_bytes<T, TJ, PA>(), &per_sm, "k_snap_y")) return -1;
+    const int nt = (inum + 31) / 32, wave = num_sms() * per_sm, ctas = (nt + NTI - 1) / NTI, rem = ctas % wave;
+    if (TJ > 4 && ctas > wave && ctas < 16 * wave && rem > 0 && 2 * rem <= wave) {
+        const int t0 = (ctas - rem) * NTI;
+        if (launch_y_part<T, TJ, PA>(yp, fp, inum, 0, t0, wave, eatom, G, s)) return -1;
+        count_launches(1);
+        return launch_y_part<T, TJ, PA>(yp, fp, inum, t0, nt - t0, wave, eatom, G, s);
+    }
+    return launch_y_part<T, TJ, PA>(yp, fp, inum, 0, nt, wave, eatom, G, s);
 }
 
 }  // namespace mdp
