@@ -159,6 +159,10 @@ template <int TJ>
 int launch_yi_pa_d(const YParams<double> &yp, ForcePath &fp, int inum, const double *G, cudaStream_t s);
 int launch_yi_full(int tj, const YParams<double> &yp, ForcePath &fp, int inum, double *eatom, const double *G,
                    cudaStream_t s);
+// Y and energies with several element types
+template <int TJ>
+int launch_y_me(const YParams<double> &yp, ForcePath &fp, int inum, int bnorm, const MeArgs &A, double *eatom,
+                cudaStream_t s);
 template <typename T, int TJ> int launch_fi(const SnapModel &m, ForcePath &fp, int inum, int nm, cudaStream_t s);
 
 // One plain-SNAP force evaluation on device data: x (anum, double4, ghosts

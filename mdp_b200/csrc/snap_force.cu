@@ -406,15 +406,7 @@ static int launch_snap_me(const SnapModel &m, ForcePath &fp, int inum, int nm, d
     fp.u_ipad = 0;
     if (rc_u) return -1;
     if (fp.timing) cudaEventRecord(fp.ev[2], s);
-    int per_sm = 0;
-    if (kernel_setup((const void *)k_snap_ei_me<TJ>, BI_WARPS * 32, 0, &per_sm, "k_snap_ei_me")) return -1;
-    k_snap_ei_me<TJ><<<std::min(A.ntiles, num_sms() * per_sm), BI_WARPS * 32, 0, s>>>(
-        fp.Ut.as<double2>(), inum, m.p.bnormflag, A, eatom);
-    const size_t sm = yi_me_smem_bytes<TJ>();
-    if (kernel_setup((const void *)k_snap_yi_me<TJ>, YI_WARPS * 32, sm, &per_sm, "k_snap_yi_me"))
-        return -1;
-    k_snap_yi_me<TJ><<<std::min(A.ntiles, num_sms() * per_sm), YI_WARPS * 32, sm, s>>>(
-        fp.Ut.as<double2>(), inum, m.yq, A, fp.Y.as<double2>());
+    if (launch_y_me<TJ>(m.yq, fp, inum, m.p.bnormflag, A, eatom, s)) return -1;
     count_launches(2);
     fp.fr_pcw = fp.pcw.as<double2>();
     const int rc_f = launch_fi<double, TJ>(m, fp, (int)nv, nm, s);
