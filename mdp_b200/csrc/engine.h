@@ -159,6 +159,9 @@ template <int TJ>
 int launch_yi_pa_d(const YParams<double> &yp, ForcePath &fp, int inum, const double *G, cudaStream_t s);
 int launch_yi_full(int tj, const YParams<double> &yp, ForcePath &fp, int inum, double *eatom, const double *G,
                    cudaStream_t s);
+// bispectrum of fp.Ut, bout[k * inum + atom]
+template <typename T, int TJ>
+int launch_b(const ForcePath &fp, int inum, int bnorm, int bzero, double *bout, cudaStream_t s);
 // Y and energies with several element types
 template <int TJ>
 int launch_y_me(const YParams<double> &yp, ForcePath &fp, int inum, int bnorm, const MeArgs &A, double *eatom,

@@ -319,8 +319,6 @@ static int launch_snap(const SnapModel &m, const YParams<T> &yp, ForcePath &fp, 
     return launch_fi<T, TJ>(m, fp, inum, nm, s);
 }
 
-int launch_bi_tiles(const double2 *Ut, int natoms, int tj, int bnorm, int bzero, double *bout, long bstride,
-                    cudaStream_t s);
 
 // Quadratic SNAP, one thread per atom: G[k][atom] = beta_k + (Q B)_k (the
 // per-atom coefficients of cpuComputeBeta2, cpuSnap.cpp:1713-1737) and
@@ -358,7 +356,7 @@ static int launch_snap_quad(const SnapModel &m, ForcePath &fp, int inum, int nm,
         return -1;
     if (launch_ui<double, TJ>(m, fp, inum, s)) return -1;
     if (fp.timing) cudaEventRecord(fp.ev[2], s);
-    if (launch_bi_tiles(fp.Ut.as<double2>(), inum, TJ, m.p.bnormflag, m.p.bzeroflag, fp.B.as<double>(), inum, s))
+    if (launch_b<double, TJ>(fp, inum, m.p.bnormflag, m.p.bzeroflag, fp.B.as<double>(), s))
         return -1;
     k_snap_quad<<<(inum + QUAD_THREADS - 1) / QUAD_THREADS, QUAD_THREADS, 0, s>>>(fp.B.as<double>(), inum, m.quad,
                                                                                fp.G.as<double>(), eatom);

@@ -644,8 +644,6 @@ int force_sq_diff(const double4 *a, const double4 *b, int n, double *dev_acc, do
 // host side
 // ---------------------------------------------------------------------------
 int launch_yi_pa_f4(const SnapModel &m, ForcePath &fp, int inum, const float *G, cudaStream_t s);
-int launch_bi_tiles_f32(const float2 *Ut, int natoms, int tj, int bnorm, int bzero, double *bout, long bstride,
-                        cudaStream_t s);
 
 int sur_features(Surrogate &S, ForcePath &fp, const double4 *x, int inum, const int *nlist, const int *nnum, int nm,
                  cudaStream_t s)
@@ -671,7 +669,7 @@ int sur_features(Surrogate &S, ForcePath &fp, const double4 *x, int inum, const 
     count_launches(2);
     if (launch_ui<float, 4>(m, fp, inum, s)) return -1;
     count_launches(1);
-    return launch_bi_tiles_f32(fp.Ut.as<float2>(), inum, 4, m.p.bnormflag, m.p.bzeroflag, S.B.as<double>(), inum, s);
+    return launch_b<float, 4>(fp, inum, m.p.bnormflag, m.p.bzeroflag, S.B.as<double>(), s);
 }
 
 int sur_force(Surrogate &S, ForcePath &fp, const double4 *x, int inum, const int *nlist, const int *nnum, int nm,
