@@ -23,6 +23,7 @@
 #include "common.cuh"
 #include "engine.h"
 #include "fit.h"
+#include "y_kernels.cuh"
 
 #include <cuda_bf16.h>
 #include <math.h>
@@ -113,22 +114,15 @@ __global__ void k_fit_zbl(const double4 *__restrict__ x, const int *__restrict__
 // Z rows of every coupling and B for j >= j1, per 32-atom tile (lane = atom)
 // Z layout [tile][zoff + (j+1) mb + ma][lane]; B layout [k][atom]
 // ---------------------------------------------------------------------------
-// Every coupling is compile-time specialised (CG coefficients as constant
-// operands, U rows in registers), output layer by layer.  Within a layer all
-// warps walk the couplings in the same order, so the code in flight is one
-// coupling's; each warp owns a row mb and a range [lo, hi) of its entries ma
-// (a plan balanced on the host), which needs no reduction between warps.
-// (Giving each warp whole (coupling, mb) rows round-robin let the warps run
-// different couplings' code at once: 4.9 no_instruction stalls per issue.)
-// warps per CTA (one CTA per SM: the 146 KB U tile): the 4,096-configuration
-// graph took 278-280 ms at 10 warps, 278 ms at 12 and 290 ms at 5
-#ifndef FIT_ZBT_WARPS_N
-#define FIT_ZBT_WARPS_N 10
-#endif
-constexpr int FIT_ZBT_WARPS = FIT_ZBT_WARPS_N;
-struct ZbPlan {
-    unsigned char mb[JD][FIT_ZBT_WARPS], lo[JD][FIT_ZBT_WARPS], hi[JD][FIT_ZBT_WARPS];   // mb 255: idle
-};
+// The jobs of the Y kernel (y_kernels.cuh): a warp takes one value of m' for all
+// layers of a parity, forms every product of two U entries once for all layers
+// of the coupling, and writes the coupling's entries when its row pairs are
+// done.  One warp per job (nine of the even layers at 2J = 8), so that no
+// entry has two owners; the right halves of the middle rows, which neither B
+// nor dB/dr reads, are not written.  Walking the couplings per output layer
+// took twice the FP64 instructions and 2.2 times the code: 1.70 ms against
+// 0.80 for 16,400 atoms at 2J = 8.
+template <int TJ> __host__ __device__ constexpr int zb_warps() { return TJ + 1; }
 
 // offset of coupling (J1, J2, J)'s rows in the Z layout (fit_tables order)
 __host__ __device__ constexpr int fit_zoff(int tj, int J1, int J2, int J)
@@ -143,84 +137,58 @@ __host__ __device__ constexpr int fit_zoff(int tj, int J1, int J2, int J)
     return -1;
 }
 
-// entries lo <= ma < hi of row mb of scale * Z_{J1 J2 J}, summed over every
-// row pair ib, written to the coupling's block Zc ([(J+1) mb + ma][lane])
-template <int J1, int J2, int J>
-__device__ __forceinline__ void zbt_rows(const int mb, const int lo, const int hi, const double2 *__restrict__ Us,
-                                         const int lane, const double scale, double2 *__restrict__ Zc)
+// the job's entries of coupling (J1, J2, J1 - J2 + 2Q..)
+template <int TJ, int J1, int J2, int Q>
+__device__ __forceinline__ void zb_write(const YSums<double, yacc_count<TJ>((J1 + J2) & 1)> &a,
+                                         double2 *__restrict__ Zt, const int top)
 {
-    constexpr int N1 = J1 + 1, N2 = J2 + 1;
-    constexpr int CGB = cg_block(J1, J2, J);
-    double yr[J + 1], yi[J + 1];
+    typedef YC<TJ, J1, J2> C;
+    if constexpr (Q < C::nj) {
+        constexpr int J = C::jlo + 2 * Q, ZO = fit_zoff(TJ, J1, J2, J), O = yacc_off(J);
+        if (J >= (top < 0 ? -top : top)) {
+            const bool mir = top > 0;
+            const int mb = (J + top) >> 1, st = mir ? -32 : 32;
+            double2 *row = Zt + (ZO + (mir ? (J + 1) * (J - mb) + J : (J + 1) * mb)) * 32;
 #pragma unroll
-    for (int ma = 0; ma <= J; ma++) { yr[ma] = 0.0; yi[ma] = 0.0; }
-    const int mb1min = max(0, (2 * mb - J - J2 + J1) / 2);
-    const int mb2max = (2 * mb - J - (2 * mb1min - J1) + J2) / 2;
-    const int nb = nb_of(J1, J2, J, mb);
-    for (int ib = 0; ib < nb; ib++) {
-        const int mb1 = mb1min + ib, mb2 = mb2max - ib;
-        const double sc = scale * cgc<double>(CGB + mb1 * N2 + mb2);
-        const double2 *r1 = Us + (idxu_block(J1) + N1 * mb1) * 32 + lane;
-        const double2 *r2 = Us + (idxu_block(J2) + N2 * mb2) * 32 + lane;
-        double u1r[N1], u1i[N1], u2r[N2], u2i[N2];
-#pragma unroll
-        for (int k = 0; k < N1; k++) { const double2 v = r1[k * 32]; u1r[k] = sc * v.x; u1i[k] = sc * v.y; }
-#pragma unroll
-        for (int k = 0; k < N2; k++) { const double2 v = r2[k * 32]; u2r[k] = v.x; u2i[k] = v.y; }
-#pragma unroll
-        for (int ma = 0; ma <= J; ma++) {
-            if (ma < lo || ma >= hi) continue;
-            const int ma1min = cmax(0, (2 * ma - J - J2 + J1) / 2);
-            const int ma2max = (2 * ma - J - (2 * ma1min - J1) + J2) / 2;
-            const int na = cmin(J1, (2 * ma - J + J2 + J1) / 2) - ma1min + 1;
-#pragma unroll
-            for (int ia = 0; ia < na; ia++) {
-                const int ma1 = ma1min + ia, ma2 = ma2max - ia;
-                const double c = cgc<double>(CGB + ma1 * N2 + ma2);
-                const double tr = c * u1r[ma1], ti = c * u1i[ma1];
-                yr[ma] += tr * u2r[ma2] - ti * u2i[ma2];
-                yi[ma] += tr * u2i[ma2] + ti * u2r[ma2];
+            for (int ma = 0; 2 * ma <= J; ma++) {
+                if (2 * ma == J && mir) continue;
+                double2 z = make_double2(a.r[O + ma], a.i[O + ma]);
+                if (mir) {
+                    if ((ma + mb) & 1) z.x = -z.x; else z.y = -z.y;
+                }
+                row[ma * st] = z;
             }
         }
+        zb_write<TJ, J1, J2, Q + 1>(a, Zt, top);
     }
-#pragma unroll
-    for (int ma = 0; ma <= J; ma++)
-        if (ma >= lo && ma < hi) Zc[(size_t)((J + 1) * mb + ma) * 32] = make_double2(yr[ma], yi[ma]);
 }
-
-template <int TJ, int J, int J1, int J2>
-__device__ __forceinline__ void zbt_layer(const double2 *__restrict__ Us, double2 *__restrict__ Zt, const int lane,
-                                          const int mb, const int lo, const int hi, const double scale)
+template <int TJ, int PAR, int J1, int J2>
+__device__ __forceinline__ void zb_couplings(const double2 *__restrict__ Us, double2 *__restrict__ Zt, const int top,
+                                             const YParams<double> &P)
 {
     if constexpr (J1 <= TJ) {
         if constexpr (J2 <= J1) {
-            if constexpr (coupling_ok(J1, J2, J)) {
-                constexpr int ZO = fit_zoff(TJ, J1, J2, J);
-                zbt_rows<J1, J2, J>(mb, lo, hi, Us, lane, scale, Zt + (size_t)ZO * 32);
+            if constexpr (((J1 + J2) & 1) == PAR) {
+                YSums<double, yacc_count<TJ>(PAR)> a;
+                a.zero();
+                int next = 0;
+                y_block<double, TJ, J1, J2>(a, Us, Us, top, YScale<double, false>{P, nullptr}, true, next, 1);
+                zb_write<TJ, J1, J2, 0>(a, Zt, top);
             }
-            zbt_layer<TJ, J, J1, J2 + 1>(Us, Zt, lane, mb, lo, hi, scale);
+            zb_couplings<TJ, PAR, J1, J2 + 1>(Us, Zt, top, P);
         } else {
-            zbt_layer<TJ, J, J1 + 1, 0>(Us, Zt, lane, mb, lo, hi, scale);
+            if constexpr (J1 >= 3) __syncthreads();   // keeps the warps in step
+            zb_couplings<TJ, PAR, J1 + 1, 0>(Us, Zt, top, P);
         }
     }
 }
 
-template <int TJ, int J>
-__device__ __forceinline__ void zbt_layers(const double2 *__restrict__ Us, double2 *__restrict__ Zt, const int lane,
-                                           const int w, const int bnorm, const ZbPlan &P)
-{
-    if constexpr (J <= TJ) {
-        const int mb = P.mb[J][w];
-        if (mb != 255) zbt_layer<TJ, J, 0, 0>(Us, Zt, lane, mb, P.lo[J][w], P.hi[J][w], bnorm ? 1.0 / (J + 1) : 1.0);
-        __syncthreads();   // keeps the warps on one layer's code
-        zbt_layers<TJ, J + 1>(Us, Zt, lane, w, bnorm, P);
-    }
-}
-
+// P: factor of each coupling in betaY (1, or 1 / (j + 1) with bnorm)
 template <int TJ>
-__global__ void __launch_bounds__(FIT_ZBT_WARPS * 32, 1)
-k_fit_zbt(const double2 *__restrict__ Ut, int natoms, const FitTables *__restrict__ T, const ZbPlan P,
-          double2 *__restrict__ Z, double *__restrict__ B, int tile_lo, int tile_hi)
+__global__ void __launch_bounds__(zb_warps<TJ>() * 32, 1)
+k_fit_zbt(const double2 *__restrict__ Ut, int natoms, const FitTables *__restrict__ T,
+          const __grid_constant__ YParams<double> P, double2 *__restrict__ Z, double *__restrict__ B, int tile_lo,
+          int tile_hi)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     double2 *Us = reinterpret_cast<double2 *>(smraw);
@@ -232,10 +200,12 @@ k_fit_zbt(const double2 *__restrict__ Ut, int natoms, const FitTables *__restric
         for (int k = threadIdx.x; k < NU * 32; k += blockDim.x) Us[k] = src[k];
         __syncthreads();
         double2 *Zt = Z + (size_t)(tile - tile_lo) * nz * 32 + lane;
-        zbt_layers<TJ, 0>(Us, Zt, lane, w, T->bnorm, P);   // ends on a barrier: B reads other warps' Z rows
+        zb_couplings<TJ, 0, 0, 0>(Us + lane, Zt, yj_top<TJ>(w), P);
+        zb_couplings<TJ, 1, 0, 0>(Us + lane, Zt, w < TJ ? yj_top<TJ>(TJ + 1 + w) : yj_none<TJ>(1), P);
+        __syncthreads();   // B reads other warps' Z rows
         // B_k = 2 sum_half w Re(U_j* Z) (- bzero), cpuComputeBi2 (cpuSnap2.cpp:516-541)
         const int atom = tile * 32 + lane;
-        for (int k = w; k < T->ntri; k += FIT_ZBT_WARPS) {
+        for (int k = w; k < T->ntri; k += zb_warps<TJ>()) {
             const FitTriple tr = T->tr[k];
             const int j = tr.j;
             const FitCoupling cp = T->cp[tr.coup[0]];
@@ -907,94 +877,21 @@ static int fit_du(mdp_fit *h, const mdp_fit::Chunk &ck)
     return tj == 8 ? fit_launch_du<8>(h, ck) : tj == 6 ? fit_launch_du<6>(h, ck) : fit_launch_du<4>(h, ck);
 }
 
-// least largest sum of c cut into k contiguous chunks (greedy under a cap)
-static long zb_min_cap(const std::vector<long> &c, int k)
-{
-    long lo = 0, hi = 0;
-    for (long v : c) { lo = std::max(lo, v); hi += v; }
-    while (lo < hi) {
-        const long mid = (lo + hi) / 2;
-        int n = 1;
-        long run = 0;
-        for (long v : c) {
-            if (run + v > mid) { n++; run = v; }
-            else run += v;
-        }
-        if (n <= k) hi = mid;
-        else lo = mid + 1;
-    }
-    return lo;
-}
-
-// The Z-kernel plan of 2J = tj: per layer J, the rows get warps where the
-// costliest chunk is, and each row's entries ma are cut into that many
-// contiguous ranges of least largest cost.  Cost of entry ma: 6 instructions
-// per term over every coupling and row pair; every warp on a row also pays
-// the row pairs' U loads (4 per u1 entry with its scaling, 1 per u2 entry).
-static ZbPlan zb_plan(int tj)
-{
-    ZbPlan P;
-    memset(&P, 0, sizeof(P));
-    memset(P.mb, 255, sizeof(P.mb));
-    for (int J = 0; J <= tj; J++) {
-        const int R = J / 2 + 1;
-        std::vector<std::vector<long>> c(R, std::vector<long>(J + 1, 0));
-        std::vector<long> load(R, 0);
-        for (int mb = 0; mb < R; mb++)
-            for (int j1 = 0; j1 <= tj; j1++)
-                for (int j2 = 0; j2 <= j1; j2++) {
-                    if (!coupling_ok(j1, j2, J)) continue;
-                    const int nb = nb_of(j1, j2, J, mb);
-                    load[mb] += (long)nb * (4 * (j1 + 1) + (j2 + 1));
-                    for (int ma = 0; ma <= J; ma++) {
-                        const int ma1min = std::max(0, (2 * ma - J - j2 + j1) / 2);
-                        const int na = std::min(j1, (2 * ma - J + j2 + j1) / 2) - ma1min + 1;
-                        c[mb][ma] += 6L * nb * na;
-                    }
-                }
-        std::vector<int> nw(R, 1);
-        for (int used = R; used < FIT_ZBT_WARPS; used++) {
-            int best = -1;
-            long bc = -1;
-            for (int r = 0; r < R; r++) {
-                if (nw[r] >= J + 1) continue;
-                const long v = zb_min_cap(c[r], nw[r]) + load[r];
-                if (v > bc) { bc = v; best = r; }
-            }
-            if (best < 0) break;
-            nw[best]++;
-        }
-        int w = 0;
-        for (int r = 0; r < R; r++) {
-            const long cap = zb_min_cap(c[r], nw[r]);
-            int a = 0;
-            for (int k = 0; k < nw[r]; k++, w++) {
-                int b = a;
-                long run = 0;
-                if (k == nw[r] - 1) b = J + 1;
-                else
-                    while (b <= J && run + c[r][b] <= cap) run += c[r][b++];
-                P.mb[J][w] = (unsigned char)r;
-                P.lo[J][w] = (unsigned char)a;
-                P.hi[J][w] = (unsigned char)b;
-                a = b;
-            }
-        }
-    }
-    return P;
-}
-
 // Z rows and B of one chunk's tiles (the fit takes 2J = 4, 6, 8)
 template <int TJ>
 static int fit_zbt(mdp_fit *h, const mdp_fit::Chunk &ck, unsigned g)
 {
-    static const ZbPlan plan = zb_plan(TJ);
+    YParams<double> P;
+    memset(&P, 0, sizeof(P));
+    for (int j1 = 0; j1 <= TJ; j1++)
+        for (int j2 = 0; j2 <= j1; j2++)
+            for (int j = j1 - j2; j <= std::min(TJ, j1 + j2); j += 2)
+                P.betaY[tri_index(j1, j2, j)] = h->tab.bnorm ? 1.0 / (j + 1) : 1.0;
     const size_t zsm = (size_t)idxu_count(TJ) * 32 * sizeof(double2);
     int per_sm = 0;
-    if (kernel_setup((const void *)k_fit_zbt<TJ>, FIT_ZBT_WARPS * 32, zsm, &per_sm, "k_fit_zbt")) return -1;
-    k_fit_zbt<TJ><<<g, FIT_ZBT_WARPS * 32, zsm, h->s>>>(h->fp.Ut.as<double2>(), h->natoms, h->tabs.as<FitTables>(),
-                                                       plan, h->Z.as<double2>(), h->B.as<double>(), ck.t_lo,
-                                                       ck.t_hi);
+    if (kernel_setup((const void *)k_fit_zbt<TJ>, zb_warps<TJ>() * 32, zsm, &per_sm, "k_fit_zbt")) return -1;
+    k_fit_zbt<TJ><<<g, zb_warps<TJ>() * 32, zsm, h->s>>>(h->fp.Ut.as<double2>(), h->natoms, h->tabs.as<FitTables>(), P,
+                                                         h->Z.as<double2>(), h->B.as<double>(), ck.t_lo, ck.t_hi);
     return 0;
 }
 
