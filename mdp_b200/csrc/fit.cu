@@ -36,41 +36,78 @@ namespace mdp {
 // ---------------------------------------------------------------------------
 // pairs: every atom against every atom of its configuration and the 27 images
 // ---------------------------------------------------------------------------
+// One warp per atom: the lanes test 32 (atom, image) candidates at a time in the
+// list's order, a ballot ranks the pairs found, and their geometry is evaluated
+// 32 pairs at a time.  (A thread per atom walks some 27 x 150 candidates one
+// after the other: 0.17 + 0.89 ms for 2,700 atoms.)
+constexpr int FIT_PAIR_WARPS = 4;
 template <bool EMIT>
-__global__ void k_fit_pairs(const double4 *__restrict__ x, const int *__restrict__ cfg, const int *__restrict__ ca0,
-                            const int *__restrict__ cn, const double4 *__restrict__ cbox, int natoms, SnapGeom gp,
-                            int *__restrict__ pcount, const int *__restrict__ poff, double4 *__restrict__ prij,
-                            double4 *__restrict__ pab, int2 *__restrict__ pinfo)
+__global__ void __launch_bounds__(FIT_PAIR_WARPS * 32)
+k_fit_pairs(const double4 *__restrict__ x, const int *__restrict__ cfg, const int *__restrict__ ca0,
+            const int *__restrict__ cn, const double4 *__restrict__ cbox, int natoms, SnapGeom gp,
+            int *__restrict__ pcount, const int *__restrict__ poff, double4 *__restrict__ prij,
+            double4 *__restrict__ pab, int2 *__restrict__ pinfo)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= natoms) return;
+    __shared__ int found[FIT_PAIR_WARPS][64];   // candidates of pairs not yet emitted
+    const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+    const int i = blockIdx.x * FIT_PAIR_WARPS + wb;
+    if (i >= natoms) return;   // whole warps leave together
     const int c = cfg[i], a0 = ca0[c], n = cn[c];
     // lattice vectors a, b, c of the configuration's cell (rows of cbox)
     const double4 la = cbox[3 * c], lb = cbox[3 * c + 1], lc = cbox[3 * c + 2], xi = x[i];
-    int cnt = 0, p = EMIT ? poff[i] : 0;
-    for (int jj = 0; jj < n; jj++) {
+    auto vec = [&](const int q, double &d0, double &d1, double &d2) {
+        const int jj = q / 27, im = q - 27 * jj;
         const double4 xj = x[a0 + jj];
-        for (int im = 0; im < 27; im++) {
-            const double u = im % 3 - 1, v = (im / 3) % 3 - 1, w = im / 9 - 1;
-            const double sx = u * la.x + v * lb.x + w * lc.x, sy = u * la.y + v * lb.y + w * lc.y,
-                         sz = u * la.z + v * lb.z + w * lc.z;
-            const double d0 = xj.x + sx - xi.x, d1 = xj.y + sy - xi.y, d2 = xj.z + sz - xi.z;
+        const double u = im % 3 - 1, v = (im / 3) % 3 - 1, w = im / 9 - 1;
+        const double sx = u * la.x + v * lb.x + w * lc.x, sy = u * la.y + v * lb.y + w * lc.y,
+                     sz = u * la.z + v * lb.z + w * lc.z;
+        d0 = xj.x + sx - xi.x;
+        d1 = xj.y + sy - xi.y;
+        d2 = xj.z + sz - xi.z;
+    };
+    int cnt = 0, p = EMIT ? poff[i] : 0, nf = 0;
+    auto emit = [&](const int m) {   // the first m <= 32 candidates of found
+        if (lane < m) {
+            const int q = found[wb][lane];
+            double d0, d1, d2;
+            vec(q, d0, d1, d2);
+            PairGeo g;
+            pair_geometry<false>(g, d0, d1, d2, gp);
+            prij[p + lane] = make_double4(d0, d1, d2, g.sfac);
+            pab[p + lane] = make_double4(g.ar, g.ai, g.br, g.bi);
+            pinfo[p + lane] = make_int2(i, a0 + q / 27);
+        }
+        p += m;
+    };
+    for (int q0 = 0; q0 < 27 * n; q0 += 32) {
+        const int q = q0 + lane;
+        bool pair = false;
+        if (q < 27 * n) {
+            double d0, d1, d2;
+            vec(q, d0, d1, d2);
             const double rsq = d0 * d0 + d1 * d1 + d2 * d2;
-            if (rsq < gp.rcutsq && rsq > 1e-20) {
-                if (EMIT) {
-                    PairGeo g;
-                    pair_geometry<false>(g, d0, d1, d2, gp);
-                    prij[p] = make_double4(d0, d1, d2, g.sfac);
-                    pab[p] = make_double4(g.ar, g.ai, g.br, g.bi);
-                    pinfo[p] = make_int2(i, a0 + jj);
-                    p++;
-                } else {
-                    cnt++;
-                }
+            pair = rsq < gp.rcutsq && rsq > 1e-20;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, pair);
+        if constexpr (EMIT) {
+            if (pair) found[wb][nf + __popc(m & ((1u << lane) - 1u))] = q;
+            nf += __popc(m);
+            __syncwarp();
+            if (nf >= 32) {
+                emit(32);
+                __syncwarp();
+                nf -= 32;
+                const int v = found[wb][32 + lane];
+                __syncwarp();
+                if (lane < nf) found[wb][lane] = v;
+                __syncwarp();
             }
+        } else {
+            cnt += __popc(m);
         }
     }
-    if (!EMIT) pcount[i] = cnt;
+    if constexpr (EMIT) emit(nf);
+    else if (lane == 0) pcount[i] = cnt;
 }
 
 // ZBL reference potential of every atom of the batch (the pair term that MDP's
@@ -481,17 +518,37 @@ __global__ void k_fit_rev_fill(const int2 *__restrict__ pinfo, long npairs, cons
     const int a = pinfo[p].y;
     rlist[roff[a] + atomicAdd(&cursor[a], 1)] = (int)p;
 }
+// One warp per atom: each entry's place is the number of smaller ones (lists
+// longer than FIT_REV_MAX: an insertion sort in place)
+constexpr int FIT_REV_MAX = 128;
 __global__ void k_fit_rev_sort(int natoms, const int *__restrict__ roff, int *__restrict__ rlist)
 {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= natoms) return;
-    const int s = roff[a], e = roff[a + 1];
-    for (int i = s + 1; i < e; i++) {
-        const int v = rlist[i];
-        int j = i - 1;
-        while (j >= s && rlist[j] > v) { rlist[j + 1] = rlist[j]; j--; }
-        rlist[j + 1] = v;
+    const int lane = threadIdx.x & 31;
+    const long a = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (a >= natoms) return;   // whole warps leave together
+    const int s = roff[a], n = roff[a + 1] - s;
+    if (n > FIT_REV_MAX) {
+        if (lane == 0)
+            for (int i = s + 1; i < s + n; i++) {
+                const int v = rlist[i];
+                int j = i - 1;
+                while (j >= s && rlist[j] > v) { rlist[j + 1] = rlist[j]; j--; }
+                rlist[j + 1] = v;
+            }
+        return;
     }
+    int val[FIT_REV_MAX / 32], to[FIT_REV_MAX / 32];
+#pragma unroll
+    for (int k = 0; k < FIT_REV_MAX / 32; k++) {
+        const int e = 32 * k + lane;
+        val[k] = e < n ? rlist[s + e] : 0;
+        to[k] = 0;
+        for (int j = 0; e < n && j < n; j++) to[k] += rlist[s + j] < val[k];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < FIT_REV_MAX / 32; k++)
+        if (32 * k + lane < n) rlist[s + to[k]] = val[k];
 }
 
 // rows of atom a: G[a][c][k] = sum_(p: j = a) dbdr - sum_(p: i = a) dbdr,
@@ -527,36 +584,51 @@ __global__ void k_fit_rows(int a_lo, int a_hi, int ntri, const int *__restrict__
     }
 }
 
-// per configuration: bi, the virial, and the energy row [we * (N, bi)] / we * E
-__global__ void k_fit_cfg(int c_lo, int c_hi, int ntri, const int *__restrict__ ca0, const int *__restrict__ cn,
-                          const int *__restrict__ poff, const double *__restrict__ B, int natoms,
-                          const double *__restrict__ dbdr, long p_lo, const double4 *__restrict__ prij,
-                          const double *__restrict__ we, const double *__restrict__ e, double *__restrict__ bi,
-                          double *__restrict__ bv, double *__restrict__ R, double *__restrict__ tgt, long erow0)
+// per configuration: bi, the virial, and the energy row [we * (N, bi)] / we * E.
+// One CTA per configuration: FIT_CFG_PARTS threads share a component's atoms
+// and pairs, in fixed strides, and their sums are added in order.  (One thread
+// per component walks every pair of the configuration: 2.26 ms for 24
+// configurations of 6,300 pairs in the mean.)
+constexpr int FIT_CFG_PARTS = 16;
+__global__ void __launch_bounds__(FIT_CFG_PARTS * FIT_KP)
+k_fit_cfg(int c_lo, int ntri, const int *__restrict__ ca0, const int *__restrict__ cn, const int *__restrict__ poff,
+          const double *__restrict__ B, int natoms, const double *__restrict__ dbdr, long p_lo,
+          const double4 *__restrict__ prij, const double *__restrict__ we, const double *__restrict__ e,
+          double *__restrict__ bi, double *__restrict__ bv, double *__restrict__ R, double *__restrict__ tgt,
+          long erow0)
 {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;   // (config, k)
-    if (t >= (long)(c_hi - c_lo) * FIT_KP) return;
-    const int c = c_lo + (int)(t / FIT_KP), k = (int)(t % FIT_KP);
+    __shared__ double part[FIT_CFG_PARTS][FIT_KP];
+    const int c = c_lo + blockIdx.x, k = threadIdx.x % FIT_KP, q = threadIdx.x / FIT_KP, kk = k - 1;
     const int a0 = ca0[c], n = cn[c];
-    double v = 0.0;
-    if (k == 0) v = (double)n;
-    if (k >= 1 && k <= ntri) {
-        const int kk = k - 1;
-        for (int a = a0; a < a0 + n; a++) v += B[(size_t)kk * natoms + a];
-        if (bi) bi[(size_t)c * ntri + kk] = v;
-        if (bv) {
-            double s[6] = {0, 0, 0, 0, 0, 0};
-            for (long p = poff[a0]; p < poff[a0 + n]; p++) {
+    const bool comp = k >= 1 && k <= ntri;
+    double s[7] = {0, 0, 0, 0, 0, 0, 0};
+    if (comp) {
+        for (int a = a0 + q; a < a0 + n; a += FIT_CFG_PARTS) s[0] += B[(size_t)kk * natoms + a];
+        if (bv)
+            for (long p = poff[a0] + q; p < poff[a0 + n]; p += FIT_CFG_PARTS) {
                 const double4 r = prij[p];
-                const long q = p - p_lo;
-                const double bx = dbdr[(3 * q) * ntri + kk], by = dbdr[(3 * q + 1) * ntri + kk],
-                             bz = dbdr[(3 * q + 2) * ntri + kk];
-                s[0] -= r.x * bx; s[1] -= r.y * by; s[2] -= r.z * bz;
-                s[3] -= r.x * by; s[4] -= r.x * bz; s[5] -= r.y * bz;
+                const double *d = dbdr + 3 * (p - p_lo) * ntri + kk;
+                const double bx = d[0], by = d[ntri], bz = d[2 * ntri];
+                s[1] -= r.x * bx; s[2] -= r.y * by; s[3] -= r.z * bz;
+                s[4] -= r.x * by; s[5] -= r.x * bz; s[6] -= r.y * bz;
             }
-            for (int q = 0; q < 6; q++) bv[((size_t)c * ntri + kk) * 6 + q] = s[q];
+    }
+    const int nv = bv ? 7 : 1;
+    for (int v = 0; v < nv; v++) {
+        __syncthreads();
+        part[q][k] = s[v];
+        __syncthreads();
+        if (q == 0) {
+            double t = part[0][k];
+            for (int m = 1; m < FIT_CFG_PARTS; m++) t += part[m][k];
+            s[v] = t;
         }
     }
+    if (q) return;
+    const double v = k == 0 ? (double)n : s[0];
+    if (comp && bi) bi[(size_t)c * ntri + kk] = v;
+    if (comp && bv)
+        for (int m = 0; m < 6; m++) bv[((size_t)c * ntri + kk) * 6 + m] = s[1 + m];
     if (R) {
         const double w = we ? we[c] : 1.0;
         R[(size_t)(erow0 + c) * FIT_KP + k] = (k <= ntri) ? w * v : 0.0;
@@ -820,13 +892,14 @@ namespace mdp {
 static int fit_pairs(mdp_fit *h)
 {
     const int n = h->natoms;
-    const int tb = 128, gb = (n + tb - 1) / tb;
+    const int tb = 128;
+    const unsigned gw = (unsigned)((n + FIT_PAIR_WARPS - 1) / FIT_PAIR_WARPS);
     if (h->pcount.ensure(sizeof(int) * n) || h->poff.ensure(sizeof(int) * (n + 1)) ||
         h->scan_tmp.ensure(sizeof(int) * scan_tmp_ints(n + 1)))
         return -1;
-    k_fit_pairs<false><<<gb, tb, 0, h->s>>>(h->x.as<double4>(), h->cfg.as<int>(), h->ca0.as<int>(), h->cn.as<int>(),
-                                            h->cbox.as<double4>(), n, h->model.geom, h->pcount.as<int>(), nullptr,
-                                            nullptr, nullptr, nullptr);
+    k_fit_pairs<false><<<gw, FIT_PAIR_WARPS * 32, 0, h->s>>>(
+        h->x.as<double4>(), h->cfg.as<int>(), h->ca0.as<int>(), h->cn.as<int>(), h->cbox.as<double4>(), n,
+        h->model.geom, h->pcount.as<int>(), nullptr, nullptr, nullptr, nullptr);
     if (exclusive_scan(h->pcount.as<int>(), h->poff.as<int>(), n, h->scan_tmp.as<int>(), h->s)) return -1;
     int np = 0;
     MDP_CUDA_TRY(cudaMemcpyAsync(&np, h->poff.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost, h->s));
@@ -838,9 +911,9 @@ static int fit_pairs(mdp_fit *h)
         fp.pab.ensure(sizeof(double4) * pc) || fp.pinfo.ensure(sizeof(int2) * pc))
         return -1;
     MDP_CUDA_TRY(cudaMemcpyAsync(fp.poff.p, h->poff.p, sizeof(int) * (n + 1), cudaMemcpyDeviceToDevice, h->s));
-    k_fit_pairs<true><<<gb, tb, 0, h->s>>>(h->x.as<double4>(), h->cfg.as<int>(), h->ca0.as<int>(), h->cn.as<int>(),
-                                           h->cbox.as<double4>(), n, h->model.geom, nullptr, h->poff.as<int>(),
-                                           fp.prij.as<double4>(), fp.pab.as<double4>(), fp.pinfo.as<int2>());
+    k_fit_pairs<true><<<gw, FIT_PAIR_WARPS * 32, 0, h->s>>>(
+        h->x.as<double4>(), h->cfg.as<int>(), h->ca0.as<int>(), h->cn.as<int>(), h->cbox.as<double4>(), n,
+        h->model.geom, nullptr, h->poff.as<int>(), fp.prij.as<double4>(), fp.pab.as<double4>(), fp.pinfo.as<int2>());
     // reverse pairs
     if (h->rcount.ensure(sizeof(int) * n) || h->roff.ensure(sizeof(int) * (n + 1)) ||
         h->cursor.ensure(sizeof(int) * n) || h->rlist.ensure(sizeof(int) * pc))
@@ -852,7 +925,7 @@ static int fit_pairs(mdp_fit *h)
     if (exclusive_scan(h->rcount.as<int>(), h->roff.as<int>(), n, h->scan_tmp.as<int>(), h->s)) return -1;
     if (h->npairs) k_fit_rev_fill<<<pb, 256, 0, h->s>>>(fp.pinfo.as<int2>(), h->npairs, h->roff.as<int>(),
                                                         h->cursor.as<int>(), h->rlist.as<int>());
-    k_fit_rev_sort<<<gb, tb, 0, h->s>>>(n, h->roff.as<int>(), h->rlist.as<int>());
+    k_fit_rev_sort<<<(unsigned)(((long)n * 32 + tb - 1) / tb), tb, 0, h->s>>>(n, h->roff.as<int>(), h->rlist.as<int>());
     count_launches(5);
     MDP_CUDA_TRY(cudaGetLastError());
     h->pairs_ready = true;
@@ -955,13 +1028,13 @@ static int fit_chunk(mdp_fit *h, const mdp_fit::Chunk &ck, bool rows, double *G,
     if (fit_zb(h, ck)) return -1;
     if (fit_du(h, ck)) return -1;
     if (fit_dbdr(h, ck, h->db_threads)) return -1;
-    const long ta = (long)(ck.a_hi - ck.a_lo) * FIT_KP, tc = (long)(ck.c_hi - ck.c_lo) * FIT_KP;
+    const long ta = (long)(ck.a_hi - ck.a_lo) * FIT_KP;
     k_fit_rows<<<(unsigned)((ta + 255) / 256), 256, 0, h->s>>>(
         ck.a_lo, ck.a_hi, h->tab.ntri, h->poff.as<int>(), h->roff.as<int>(), h->rlist.as<int>(), h->dbdr.as<double>(),
         ck.p_lo, h->cfg.as<int>(), h->wf.as<double>(), h->f.as<double>(), G, rows ? h->R.as<double>() : nullptr,
         rows ? h->tgt.as<double>() : nullptr, h->nconf);
-    k_fit_cfg<<<(unsigned)((tc + 255) / 256), 256, 0, h->s>>>(
-        ck.c_lo, ck.c_hi, h->tab.ntri, h->ca0.as<int>(), h->cn.as<int>(), h->poff.as<int>(), h->B.as<double>(), n,
+    k_fit_cfg<<<(unsigned)(ck.c_hi - ck.c_lo), FIT_CFG_PARTS * FIT_KP, 0, h->s>>>(
+        ck.c_lo, h->tab.ntri, h->ca0.as<int>(), h->cn.as<int>(), h->poff.as<int>(), h->B.as<double>(), n,
         h->dbdr.as<double>(), ck.p_lo, h->fp.prij.as<double4>(), h->we.as<double>(), h->e.as<double>(), bi, bv,
         rows ? h->R.as<double>() : nullptr, rows ? h->tgt.as<double>() : nullptr, 0);
     count_launches(2);
