@@ -1,8 +1,9 @@
 """GPU: force stages at the sizes where their work split changes.
 
 The Y kernel gives a tile's couplings to one CTA or shares them among up to
-eight (few tiles), and its FP32 form puts two tiles in a CTA; ragged atom
-counts leave lanes, or a CTA's second tile, empty.  Energies, forces and
+eight (few tiles, or few in the last wave), and its FP32 form puts two tiles in
+a CTA; ragged atom counts leave lanes, or a CTA's second tile, empty.  The U
+kernel gives an atom's pairs to four lanes (few tiles) or one.  Energies, forces and
 virials against the oracle: FP64 within 1e-12 of the largest entry (sums of
 about 4e4 terms at 1e-16 each, some 2e-14 with random signs, times the
 cancellation of a force sum), FP32 forces within 1e-5 of it.
@@ -22,7 +23,8 @@ SIZES = [
     ((4, 4, 5), 31),      # five tiles less 31 atoms: 129 atoms
     ((9, 9, 9), 2),       # three groups (FP64)
     ((10, 11, 11), 37),   # 75 tiles: one group (FP64), the FP32 CTA's second tile missing
-    ((14, 14, 13), 40),   # 158 tiles: one group in both precisions
+    ((14, 14, 13), 40),   # 158 tiles: one group, FP64's last ten tiles a wave of their own
+    ((17, 17, 17), 3),    # 307 tiles: the same in FP32
 ]
 
 
@@ -73,3 +75,37 @@ def test_neighbour_rows_at_their_capacity(cuda_lib, cells, vac, jitter):
             assert np.array_equal(out["neighlist"][i, :nn[i]], np.sort(nl[i, :nn[i]]))
         with pytest.raises(_lib.MdpError, match="overflow"):
             snap_compute(p, x, cfg.box, skin, nm - 1)
+
+
+def replicate(x, box, reps):
+    """reps copies of a cell along its axes; the copies of an atom stay apart by n."""
+    i = np.stack(np.meshgrid(*[np.arange(r) for r in reps], indexing="ij"), -1).reshape(-1, 1, 3)
+    return np.ascontiguousarray((x[None] + i * box).reshape(-1, 3)), box * np.asarray(reps)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("kind,reps,tj", [("crystal", (8, 8, 7), 8), ("crystal", (10, 8, 10), 6), ("gas", (17, 16, 16), 8)])
+def test_large_systems_repeat_their_cell(cuda_lib, kind, reps, tj, precision):
+    """Above the size from which dE/dr runs as one sweep: a cell repeated to more
+    than 49,152 (2J = 6 FP32: 98,304) atoms has the cell's energies, forces and
+    virials in every copy.  The gas, a pair or two per atom, makes a window of
+    pairs span several turns of staged atoms, with pairless atoms between."""
+    from mdp_b200.snap import snap_compute
+    p = configs.snap_params(tj, seed=11)
+    if kind == "crystal":
+        x, box = crystal((4, 4, 4), 1, 5)
+    else:
+        rng = np.random.default_rng(3)
+        box = np.full(3, 13.0)
+        x = box * rng.random((12, 3))
+    xa, al, nl, nn = oracle.neighbor_list(x, box, p.rcut, 1.0, 80)
+    want = oracle.snap_force(xa, al, nl, nn, p)
+    xs, boxs = replicate(x, box, reps)
+    assert xs.shape[0] > (98304 if tj == 6 else 49152)
+    out = snap_compute(p, xs, boxs, 1.0, 80, precision=precision)
+    tol = 1e-12 if precision == "fp64" else 1e-5
+    # coordinates of a copy carry the rounding of the box they lie in
+    tol = max(tol, 1e-15 * max(boxs) * 30)
+    for got, ref in zip((out["eatom"], out["fatom"], out["vatom"].T), (want[0], want[1], want[2].T)):
+        ref = np.tile(ref, (xs.shape[0] // x.shape[0],) + (1,) * (ref.ndim - 1))
+        assert np.abs(got - ref).max() < tol * np.abs(ref).max()
