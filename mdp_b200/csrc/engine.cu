@@ -708,11 +708,11 @@ static int compute_device(const mdp_snap_params *p, int precision, const double 
     const int tb = 256, gb = (inum + tb - 1) / tb;
     MDP_CUDA_TRY(cudaMemsetAsync(os.nb.rcount.p, 0, sizeof(int) * inum, s));
     const unsigned gs = (unsigned)(((long)inum * neighmax + tb - 1) / tb);   // one thread per slot
-    k_rev_count<<<gs, tb, 0, s>>>(neighlist, neighnum, alist, inum, neighmax, os.nb.rcount.as<int>());
+    if (gs) k_rev_count<<<gs, tb, 0, s>>>(neighlist, neighnum, alist, inum, neighmax, os.nb.rcount.as<int>());
     if (exclusive_scan(os.nb.rcount.as<int>(), os.nb.roff.as<int>(), inum, os.nb.scan_tmp.as<int>(), s)) return -1;
     MDP_CUDA_TRY(cudaMemsetAsync(os.nb.cursor.p, 0, sizeof(int) * inum, s));
-    k_rev_fill<<<gs, tb, 0, s>>>(neighlist, neighnum, alist, inum, neighmax, os.nb.roff.as<int>(),
-                                 os.nb.cursor.as<int>(), os.nb.rlist.as<long long>());
+    if (gs) k_rev_fill<<<gs, tb, 0, s>>>(neighlist, neighnum, alist, inum, neighmax, os.nb.roff.as<int>(),
+                                         os.nb.cursor.as<int>(), os.nb.rlist.as<long long>());
     k_rev_sort<<<std::min((inum + 7) / 8, num_sms() * 8), 256, 0, s>>>(inum, os.nb.roff.as<int>(), os.nb.rlist.as<long long>());
     if (force_compute(os.fp, os.model, precision, os.x4.as<double4>(), inum, neighlist, neighnum, neighmax,
                       (long)inum * neighmax, os.nb.roff.as<int>(), os.nb.rlist.as<long long>(), eatom,

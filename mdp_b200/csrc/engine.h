@@ -25,14 +25,9 @@ __global__ void k_ghost_count(const double4 *, int, const __grid_constant__ BoxP
 __global__ void k_ghost_emit(double4 *, int *, int, const __grid_constant__ BoxParams, const int *, const unsigned *);
 __global__ void k_cell_index(const double4 *, int, const __grid_constant__ BoxParams, int *, int *);
 __global__ void k_cell_fill(int, const int *, const int *, int *, int *);
-// warps per CTA of k_neigh_build and the ints each keeps for a row of nm slots
-constexpr int NEIGH_WARPS = 4;
-__host__ __device__ inline int neigh_capacity(int nm)
-{
-    int p = 2;
-    while (p < nm) p <<= 1;
-    return p;
-}
+// warps per CTA of k_neigh_build, and the longest row (48 KB for the warps of a
+// CTA) that a warp collects and sorts in shared memory; longer ones in place
+constexpr int NEIGH_WARPS = 4, NEIGH_SHARED = 3072;
 __global__ void k_neigh_build(const double4 *, int, const __grid_constant__ BoxParams, const int *, const int *,
                               const int *, double, int, int *, int *, int *);
 __global__ void k_rev_count(const int *, const int *, const int *, int, int, int *);

@@ -215,7 +215,7 @@ __global__ void k_cell_fill(int anum, const int *__restrict__ cidx, const int *_
 // three cells along the first axis are adjacent in the cell order, so an atom's
 // 27 cells are nine ranges of catoms; the lanes test 32 candidates at a time, a
 // ballot ranks the neighbours found, and a bitonic network in shared memory
-// (row capacity rounded up to a power of two, per warp) sorts them.  A thread
+// (rows of more than NEIGH_SHARED slots: in place) sorts them.  A thread
 // per atom, with an insertion sort of the row in global memory, is a chain of
 // some 350 dependent candidate loads: 240 us for 128 atoms.
 __global__ void __launch_bounds__(NEIGH_WARPS * 32)
@@ -227,7 +227,7 @@ k_neigh_build(const double4 *__restrict__ x, int inum, const __grid_constant__ B
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * NEIGH_WARPS + w;
     if (i >= inum) return;   // whole warps leave together
-    int *buf = nbuf + w * neigh_capacity(nm);
+    int *buf = nm <= NEIGH_SHARED ? nbuf + w * nm : nlist + (size_t)i * nm;
     const double4 xi = x[i];
     const int c = cidx[i];
     const int c0 = c % bp.nc[0], c1 = (c / bp.nc[0]) % bp.nc[1], c2 = c / (bp.nc[0] * bp.nc[1]);
@@ -258,22 +258,23 @@ k_neigh_build(const double4 *__restrict__ x, int inum, const __grid_constant__ B
         if (lane == 0) atomicOr(status, 1);
         cnt = nm;
     }
-    int P = 2;
-    while (P < cnt) P <<= 1;
-    for (int k = cnt + lane; k < P; k += 32) buf[k] = INT_MAX;
+    // bitonic merge sort whose comparators all leave the smaller entry in front:
+    // those that reach past the row's end find nothing to do, so no padding
     __syncwarp();
-    for (int k = 2; k <= P; k <<= 1)
+    for (int k = 2; k < 2 * cnt; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int a = lane; a < P; a += 32) {
-                const int b = a ^ j;
-                if (b > a) {
+            const int flip = 2 * j == k ? k - 1 : j;
+            for (int a = lane; a < cnt; a += 32) {
+                const int b = a ^ flip;
+                if (b > a && b < cnt) {
                     const int u = buf[a], v = buf[b];
-                    if ((u > v) == ((a & k) == 0)) { buf[a] = v; buf[b] = u; }
+                    if (u > v) { buf[a] = v; buf[b] = u; }
                 }
             }
             __syncwarp();
         }
-    for (int k = lane; k < cnt; k += 32) nlist[(size_t)i * nm + k] = buf[k];
+    if (nm <= NEIGH_SHARED)
+        for (int k = lane; k < cnt; k += 32) nlist[(size_t)i * nm + k] = buf[k];
     if (lane == 0) nnum[i] = cnt;
 }
 

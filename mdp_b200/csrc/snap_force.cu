@@ -583,18 +583,18 @@ int neighbor_build(Neighbors &nb, const BoxParams &bp, double4 *x, int inum, dou
     k_cell_fill<<<(anum + tb - 1) / tb, tb, 0, s>>>(anum, nb.cidx.as<int>(), nb.cstart.as<int>(), nb.cursor.as<int>(),
                                                     nb.catoms.as<int>());
     MDP_CUDA_TRY(cudaMemsetAsync(nb.status.p, 0, sizeof(int), s));
-    k_neigh_build<<<(inum + NEIGH_WARPS - 1) / NEIGH_WARPS, NEIGH_WARPS * 32,
-                    sizeof(int) * NEIGH_WARPS * neigh_capacity(nm), s>>>(x, inum, bp, nb.cidx.as<int>(), nb.cstart.as<int>(),
-                                                     nb.catoms.as<int>(), rc * rc, nm, nb.nlist.as<int>(),
-                                                     nb.nnum.as<int>(), nb.status.as<int>());
+    const size_t nsm = nm <= NEIGH_SHARED ? sizeof(int) * NEIGH_WARPS * nm : 0;
+    k_neigh_build<<<(inum + NEIGH_WARPS - 1) / NEIGH_WARPS, NEIGH_WARPS * 32, nsm, s>>>(
+        x, inum, bp, nb.cidx.as<int>(), nb.cstart.as<int>(), nb.catoms.as<int>(), rc * rc, nm, nb.nlist.as<int>(),
+        nb.nnum.as<int>(), nb.status.as<int>());
     MDP_CUDA_TRY(cudaMemsetAsync(nb.rcount.p, 0, sizeof(int) * inum, s));
     const unsigned gs = (unsigned)(((long)inum * nm + tb - 1) / tb);   // one thread per slot
-    k_rev_count<<<gs, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum,
-                                                    nm, nb.rcount.as<int>());
+    if (gs) k_rev_count<<<gs, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum, nm,
+                                          nb.rcount.as<int>());
     if (exclusive_scan(nb.rcount.as<int>(), nb.roff.as<int>(), inum, tmp, s)) return -1;
     MDP_CUDA_TRY(cudaMemsetAsync(nb.cursor.p, 0, sizeof(int) * inum, s));
-    k_rev_fill<<<gs, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum, nm,
-                                                   nb.roff.as<int>(), nb.cursor.as<int>(), nb.rlist.as<long long>());
+    if (gs) k_rev_fill<<<gs, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum, nm,
+                                         nb.roff.as<int>(), nb.cursor.as<int>(), nb.rlist.as<long long>());
     k_rev_sort<<<std::min((inum + 7) / 8, num_sms() * 8), 256, 0, s>>>(inum, nb.roff.as<int>(), nb.rlist.as<long long>());
     count_launches(8);
     int hs[2] = {0, 0};

@@ -77,6 +77,20 @@ def test_neighbour_rows_at_their_capacity(cuda_lib, cells, vac, jitter):
             snap_compute(p, x, cfg.box, skin, nm - 1)
 
 
+@pytest.mark.parametrize("nm", [3072, 3073, 5000])
+def test_long_neighbour_rows(cuda_lib, nm):
+    """Rows longer than a warp's shared memory holds are collected and sorted in place."""
+    from mdp_b200.snap import snap_compute
+    p = configs.snap_params(4, seed=11)
+    x, box = crystal((3, 3, 4), 2, 7)
+    want = snap_compute(p, x, box, 1.0, 128, want_neighbors=True)
+    out = snap_compute(p, x, box, 1.0, nm, want_neighbors=True)
+    assert np.array_equal(out["neighnum"], want["neighnum"])
+    for i, n in enumerate(want["neighnum"]):
+        assert np.array_equal(out["neighlist"][i, :n], want["neighlist"][i, :n])
+    assert np.array_equal(out["fatom"], want["fatom"])
+
+
 def replicate(x, box, reps):
     """reps copies of a cell along its axes; the copies of an atom stay apart by n."""
     i = np.stack(np.meshgrid(*[np.arange(r) for r in reps], indexing="ij"), -1).reshape(-1, 1, 3)
