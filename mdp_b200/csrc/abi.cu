@@ -317,10 +317,10 @@ int ref_snap_ui(double *ur, double *ui, const double *rij, double rcut, double w
     {                                                                                                              \
         const size_t sm = (size_t)UI_WARPS * (idxu_count(TJ) + 32 * (TJ + 1)) * sizeof(double2);                  \
         int per_sm = 0;                                                                                            \
-        if (kernel_setup((const void *)k_snap_ui<double, TJ, true>, UI_WARPS * 32, sm, &per_sm, "k_snap_ui"))      \
+        if (kernel_setup((const void *)k_snap_ui<double, TJ>, UI_WARPS * 32, sm, &per_sm, "k_snap_ui"))            \
             return -1;                                                                                             \
-        k_snap_ui<double, TJ, true><<<blocks, UI_WARPS * 32, sm, s>>>(c.off.as<int>(), c.fp.prij.as<double4>(),    \
-                                                                      inum, c.model.geom, nullptr, ur, ui);        \
+        k_snap_ui<double, TJ><<<blocks, UI_WARPS * 32, sm, s>>>(c.off.as<int>(), c.fp.prij.as<double4>(),          \
+                                                                inum, c.model.geom, ur, ui);                       \
     }
     switch (tj) {
     case 4: MDP_UIREF(4) break;
@@ -604,11 +604,11 @@ int ref_snap_ui_me(double *ur, double *ui, const double *rij, const double *rade
     {                                                                                                              \
         const size_t sm = (size_t)UI_WARPS * (idxu_count(TJ) + 32 * (TJ + 1)) * sizeof(double2);                  \
         int per_sm = 0;                                                                                            \
-        if (kernel_setup((const void *)k_snap_ui<double, TJ, true>, UI_WARPS * 32, sm, &per_sm, "k_snap_ui"))      \
+        if (kernel_setup((const void *)k_snap_ui<double, TJ>, UI_WARPS * 32, sm, &per_sm, "k_snap_ui"))            \
             return -1;                                                                                             \
-        k_snap_ui<double, TJ, true><<<blocks, UI_WARPS * 32, sm, s>>>(c.off.as<int>(), c.fp.prij.as<double4>(),    \
-                                                                      (int)nv, c.model.geom, nullptr, ur, ui,      \
-                                                                      c.fp.pcw.as<double2>(), inum);              \
+        k_snap_ui<double, TJ><<<blocks, UI_WARPS * 32, sm, s>>>(c.off.as<int>(), c.fp.prij.as<double4>(),          \
+                                                                (int)nv, c.model.geom, ur, ui,                     \
+                                                                c.fp.pcw.as<double2>(), inum);                     \
     }
     switch (tj) {
     case 4: MDP_UIREF_ME(4) break;

@@ -65,7 +65,6 @@ const char *get_error();
 // Every translation unit that launches SNAP kernels holds its own copy and
 // fills it through tu_ensure_tables() before its first launch on a device.
 static __constant__ double c_rootpq_d[JD * JD];
-static __constant__ float c_rootpq_f[JD * JD];
 // unorm[(J*JD + mb)*JD + ma] = sqrt(ma! (J-ma)! / ((J-mb)! mb!)): the factor
 // between a U entry of row mb, layer J and its coefficient-free form (below)
 static __constant__ double c_unorm_d[JD * JD * JD];
@@ -77,17 +76,15 @@ static __constant__ float c_cg_f[NCG];
 static int tu_fill_tables()
 {
     static double cg[NCG], rp[JD * JD], un[JD * JD * JD];
-    static float cgf[NCG], rpf[JD * JD], unf[JD * JD * JD];
+    static float cgf[NCG], unf[JD * JD * JD];
     host_cg_table(cg);
     host_rootpq_table(rp);
     host_unorm_table(un);
     for (int i = 0; i < NCG; i++) cgf[i] = (float)cg[i];
-    for (int i = 0; i < JD * JD; i++) rpf[i] = (float)rp[i];
     for (int i = 0; i < JD * JD * JD; i++) unf[i] = (float)un[i];
     if (cudaMemcpyToSymbol(c_cg_d, cg, sizeof(cg)) != cudaSuccess ||
         cudaMemcpyToSymbol(c_cg_f, cgf, sizeof(cgf)) != cudaSuccess ||
         cudaMemcpyToSymbol(c_rootpq_d, rp, sizeof(rp)) != cudaSuccess ||
-        cudaMemcpyToSymbol(c_rootpq_f, rpf, sizeof(rpf)) != cudaSuccess ||
         cudaMemcpyToSymbol(c_unorm_d, un, sizeof(un)) != cudaSuccess ||
         cudaMemcpyToSymbol(c_unorm_f, unf, sizeof(unf)) != cudaSuccess) {
         set_error("uploading SNAP constant tables failed");
@@ -127,7 +124,6 @@ template <> struct cplx<float> { typedef float2 type; };
 
 template <typename T> __device__ __forceinline__ T rootpq(int p, int q);
 template <> __device__ __forceinline__ double rootpq<double>(int p, int q) { return c_rootpq_d[p * JD + q]; }
-template <> __device__ __forceinline__ float rootpq<float>(int p, int q) { return c_rootpq_f[p * JD + q]; }
 
 template <typename T> __device__ __forceinline__ T unorm(int j, int mb, int ma);
 template <> __device__ __forceinline__ double unorm<double>(int j, int mb, int ma) { return c_unorm_d[(j * JD + mb) * JD + ma]; }

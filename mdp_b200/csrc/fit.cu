@@ -14,7 +14,7 @@
 //
 // Pipeline (all on one stream, captured into one CUDA graph by mdp_fit_run):
 //   pairs (brute force over each configuration's atoms and 27 images)
-//   U      (k_snap_uc, the MD engine's kernel)
+//   U      (k_snap_ur, the MD engine's kernel)
 //   Z, B   (k_fit_zbt: every coupling's Z rows per atom, B for j >= j1)
 //   dU/dr  (k_fit_du: forward-mode, coefficient-free recursion, per pair and direction)
 //   dB/dr  (k_fit_dbdr: the three Z . dU terms of cpuComputeDbidrj:826-1013)

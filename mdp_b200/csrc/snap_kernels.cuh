@@ -2,20 +2,24 @@
 // (double: plain path; float: reduced-precision form) and on 2J (TJ).
 //
 // Stages (reference functions in src/C++/Core/cpuSnap4.cpp):
-//   k_snap_ui   U_i = sum_j sfac(r_ij) U(r_ij) + wself, mirrored   (:11-244)
-//               one warp per atom, lanes over its pairs, per-row
+//   k_snap_ur   U_i = sum_j sfac(r_ij) U(r_ij) + wself, mirrored   (:11-244)
+//               (u_kernels.cuh)
+//   k_snap_ui   the same sum in the reference's layout (the stage entry
+//               points): one warp per atom, lanes over its pairs, per-row
 //               shared-memory transpose to sum the lanes
 //   k_snap_y    Y_i = sum_{j1 j2} beta' Z_{j1 j2 j}(U_i)  and
 //               E_i = beta0 + 2/3 sum_half w Re(U* Y)        (:250-421, :697-792)
 //               (y_kernels.cuh)
 //   k_snap_yi   the same for a U that need not have the inversion symmetry (the
-//               stage entry points), FP64: tiles of 32 atoms (lane = atom), U
-//               tile resident in shared memory, every (j1,j2,j) row of Z specialised at compile time
-//               so CG coefficients are constant-bank operands and the U rows
-//               it needs are held in registers
+//               stage entry points), FP64: tiles of 32 atoms (lane = atom), the
+//               U tile in shared memory, every (j1,j2,j) row of Z specialised
+//               at compile time: CG coefficients are constant-bank operands
+//               and the U rows a row needs are held in registers
 //   k_snap_fr   dE/dr_ij = 2 sum_half w Re(Y* dU/dr)         (:798-1175)
 //               one thread per pair, reverse-mode (adjoint) differentiation
 //               of the U recursion seeded with Y
+//   k_snap_fc   the same by one forward sweep and four sums, for many atoms
+//               (f_kernels.cuh)
 #pragma once
 
 #include "common.cuh"
@@ -169,21 +173,20 @@ __device__ __forceinline__ void u_rows(const T ar, const T ai, const T br, const
 }
 
 // ---------------------------------------------------------------------------
-// k_snap_ui: warp per atom.  Output U in 32-atom tiles: Ut[tile][k][lane],
-// k = idxu index (full plane, wself added and mirrored).
+// k_snap_ui: warp per atom.  U of the stage entry points: the computed rows
+// (no wself, no mirror) are added into the reference's layout
+// Ur/Ui[k * natoms + atom] (cpuSnapComputeUi, cpuSnap4.cpp:11-187)
 // ---------------------------------------------------------------------------
 constexpr int UI_WARPS = 4;
 
-// REF = true: no wself/mirror; the computed rows are added into the reference's
-// layout Ur/Ui[k * natoms + atom] (cpuSnapComputeUi semantics, cpuSnap4.cpp:11-187)
 // With pcw, each pair's cutoff and neighbour weight come from pcw[p]; with
 // iblk, atom i is row i % iblk of element block i / iblk of the reference's
 // [block][k][iblk] layout (chemflag U, cpuSnap4.cpp:59-61).
-template <typename T, int TJ, bool REF = false>
+template <typename T, int TJ>
 __global__ void __launch_bounds__(UI_WARPS * 32)
 k_snap_ui(const int *__restrict__ poff, const double4 *__restrict__ prij, int natoms, SnapGeom gp,
-          typename cplx<T>::type *__restrict__ Ut, double *__restrict__ Uref_r = nullptr,
-          double *__restrict__ Uref_i = nullptr, const double2 *__restrict__ pcw = nullptr, int iblk = 0)
+          double *__restrict__ Uref_r, double *__restrict__ Uref_i, const double2 *__restrict__ pcw = nullptr,
+          int iblk = 0)
 {
     typedef typename cplx<T>::type T2;
     constexpr int NU = idxu_count(TJ);
@@ -233,39 +236,17 @@ k_snap_ui(const int *__restrict__ poff, const double4 *__restrict__ prij, int na
         for (int o = 16; o > 0; o >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, o);
         if (lane == 0) acc[0].x += ssum;
         __syncwarp();
-        if constexpr (REF) {
-            const int nrow = iblk > 0 ? iblk : natoms;
-            const size_t base = (size_t)(i / nrow) * NU * nrow + (i % nrow);
-            for (int k = lane; k < NU; k += 32) {
-                int j = 0;
-                while (idxu_block(j + 1) <= k) j++;
-                const int mb = (k - idxu_block(j)) / (j + 1);
-                if (2 * mb <= j) {
-                    Uref_r[base + (size_t)k * nrow] += (double)acc[k].x;
-                    Uref_i[base + (size_t)k * nrow] += (double)acc[k].y;
-                }
-            }
-            __syncwarp();
-            continue;
-        }
-        // wself = 1 on the diagonal of the computed half (cpuAddWself2Ui)
-        for (int j = lane; j <= TJ; j += 32)
-            for (int m = 0; 2 * m <= j; m++) acc[idxu_block(j) + (j + 1) * m + m].x += T(1);
-        __syncwarp();
-        // mirror rows mb < j/2 into rows j-mb: U(j-mb, j-ma) = (-1)^(ma+mb) conj U(mb, ma)
+        const int nrow = iblk > 0 ? iblk : natoms;
+        const size_t base = (size_t)(i / nrow) * NU * nrow + (i % nrow);
         for (int k = lane; k < NU; k += 32) {
             int j = 0;
             while (idxu_block(j + 1) <= k) j++;
-            const int rem = k - idxu_block(j), mb = rem / (j + 1), ma = rem - mb * (j + 1);
-            if (2 * mb < j) {
-                const T s = ((ma + mb) & 1) ? T(-1) : T(1);
-                const T2 v = acc[k];
-                acc[idxu_block(j) + (j + 1) * (j - mb) + (j - ma)] = T2{s * v.x, -s * v.y};
+            const int mb = (k - idxu_block(j)) / (j + 1);
+            if (2 * mb <= j) {
+                Uref_r[base + (size_t)k * nrow] += (double)acc[k].x;
+                Uref_i[base + (size_t)k * nrow] += (double)acc[k].y;
             }
         }
-        __syncwarp();
-        T2 *dst = Ut + (size_t)(i >> 5) * NU * 32 + (i & 31);
-        for (int k = lane; k < NU; k += 32) dst[(size_t)k * 32] = acc[k];
         __syncwarp();
     }
 }
@@ -329,16 +310,6 @@ __device__ __forceinline__ void cf_fwd(const T ar, const T ai, const T br, const
     }
 }
 
-// the half plane without the entries right of a middle row's centre (the mirror
-// of its left half): 145 entries at 2J = 8 against 155
-__host__ __device__ constexpr int uh_len(int j) { return (j + 1) * ((j + 1) / 2) + (j % 2 == 0 ? j / 2 + 1 : 0); }
-__host__ __device__ constexpr int uh_block(int j)
-{
-    int n = 0;
-    for (int jj = 0; jj < j; jj++) n += uh_len(jj);
-    return n;
-}
-__host__ __device__ constexpr int uh_count(int tj) { return uh_block(tj + 1); }
 // ---------------------------------------------------------------------------
 // k_snap_yi
 // ---------------------------------------------------------------------------
@@ -355,9 +326,7 @@ __host__ __device__ constexpr int items_of(int j1, int j2, int j)
     return n;
 }
 
-// One warp's partial output row of a layer, in registers: separate real and
-// imaginary parts in FP64; {re, im} pairs in FP32, where the packed two-lane
-// instructions of sm_100 do the complex arithmetic.
+// One warp's partial output row of a layer, in registers
 template <typename T> struct YRow {
     T r[JD], i[JD];
     __device__ __forceinline__ void zero()
@@ -367,62 +336,6 @@ template <typename T> struct YRow {
     }
     __device__ __forceinline__ typename cplx<T>::type get(int m) const { return {r[m], i[m]}; }
 };
-template <> struct YRow<float> {
-    float2 v[JD];
-    __device__ __forceinline__ void zero()
-    {
-#pragma unroll
-        for (int m = 0; m < JD; m++) v[m] = make_float2(0.f, 0.f);
-    }
-    __device__ __forceinline__ float2 get(int m) const { return v[m]; }
-};
-
-// FP32 rows: for every (ma1, ma2) the product p = (s u1[ma1]) u2[ma2] takes a
-// packed multiply and a packed fused multiply-add ({ar, ai} * {br, br}, then
-// {-ai, ar} * {bi, bi} added), and y[ma] += c p one more packed FMA, with
-// ma = ma1 + ma2 - (J1 + J2 - J)/2.  u2 stays in registers as {re, re} and
-// {im, im}; u1 streams from shared memory one entry at a time.
-template <int J1, int J2, int J>
-__device__ __forceinline__ void z_rows_f32(const int mb, const int o, const int st, const float2 *__restrict__ Us,
-                                           const float2 *__restrict__ Us2, const int lane, const float beta,
-                                           YRow<float> &acc)
-{
-    constexpr int N1 = J1 + 1, N2 = J2 + 1;
-    constexpr int CGB = cg_block(J1, J2, J);
-    constexpr int OFF = (J1 + J2 - J) / 2;
-    const int mb1min = max(0, (2 * mb - J - J2 + J1) / 2);
-    const int mb2max = (2 * mb - J - (2 * mb1min - J1) + J2) / 2;
-    const int nb = min(J1, (2 * mb - J + J2 + J1) / 2) - mb1min + 1;
-    for (int ib = o; ib < nb; ib += st) {
-        const int mb1 = mb1min + ib, mb2 = mb2max - ib;
-        const float s = beta * cgc<float>(CGB + mb1 * N2 + mb2);
-        const float2 *r1 = Us + (idxu_block(J1) + N1 * mb1) * 32 + lane;
-        const float2 *r2 = Us2 + (idxu_block(J2) + N2 * mb2) * 32 + lane;
-        float2 br[N2], bi[N2];
-#pragma unroll
-        for (int a = 0; a < N2; a++) {
-            const float2 v = r2[a * 32];
-            br[a] = make_float2(v.x, v.x);
-            bi[a] = make_float2(v.y, v.y);
-        }
-#pragma unroll
-        for (int ma1 = 0; ma1 < N1; ma1++) {
-            const float2 v = r1[ma1 * 32];
-            const float2 a = __fmul2_rn(make_float2(s, s), v);
-            const float2 an = make_float2(-a.y, a.x);
-#pragma unroll
-            for (int ma2 = 0; ma2 < N2; ma2++) {
-                const int ma = ma1 + ma2 - OFF;
-                if (ma < 0 || ma > J) continue;
-                float2 p = __fmul2_rn(a, br[ma2]);
-                p = __ffma2_rn(an, bi[ma2], p);
-                const float c = cgc<float>(CGB + ma1 * N2 + ma2);
-                acc.v[ma] = __ffma2_rn(make_float2(c, c), p, acc.v[ma]);
-            }
-        }
-    }
-}
-
 // Row mb of beta' Z_{J1 J2 J}, restricted to the row pairs ib = o, o+st, ...,
 // accumulated into the warp's row (registers).  The J1 factor is read from
 // Us, the J2 factor from Us2 (the same tile for one element; the U blocks of
@@ -433,10 +346,6 @@ __device__ __forceinline__ void z_rows(const int mb, const int o, const int st,
                                        const typename cplx<T>::type *__restrict__ Us2, const int lane, const T beta,
                                        YRow<T> &acc)
 {
-    if constexpr (std::is_same<T, float>::value) {
-        z_rows_f32<J1, J2, J>(mb, o, st, Us, Us2, lane, beta, acc);
-        return;
-    } else {
     T(&yr)[JD] = acc.r;
     T(&yi)[JD] = acc.i;
     typedef typename cplx<T>::type T2;
@@ -469,7 +378,6 @@ __device__ __forceinline__ void z_rows(const int mb, const int o, const int st,
                 yi[ma] += tr * u2i[ma2] + ti * u2r[ma2];
             }
         }
-    }
     }
 }
 
