@@ -80,10 +80,12 @@ def fr_flops_per_pair(tj):
     return fl
 
 
-# algorithmic FLOPs (2J=8), per atom or pair: Z/Y 41,889 complex terms x 11
-# and energy 1,413 x 4 (the reference's minimal contraction count), U 154
-# half-plane elements x 22 per pair, dE/dr as implemented (reverse mode)
-FLOP_Y_PER_ATOM = 41889 * 11 + 1413 * 4
+# algorithmic FLOPs (2J=8), per atom or pair: Y as implemented (every product of
+# two U entries once: 14,880 complex products, 39,977 of them times a real
+# coefficient added to a layer's sum, 8,712 of those sums scaled and added to Y)
+# and the energy's 155 x 4; U 154 half-plane elements x 22 per pair (the
+# reference's recursion), dE/dr as implemented (reverse mode)
+FLOP_Y_PER_ATOM = 14880 * 6 + 39977 * 4 + 8712 * 4 + 155 * 4
 FLOP_U_PER_PAIR = 154 * 22
 FLOP_F_PER_PAIR = fr_flops_per_pair(8)
 
@@ -492,7 +494,7 @@ def run_ours(args):
             ref_gpu = {"error": str(ex)[:200]}
 
     traffic = None
-    prof = os.path.join(HERE, "profiles", "k_snap_yi_fp64_traffic.json")
+    prof = os.path.join(HERE, "profiles", "k_snap_y_fp64_traffic.json")
     if os.path.exists(prof):
         with open(prof) as fh:
             tr = json.load(fh)
@@ -512,7 +514,7 @@ def run_ours(args):
             "e2e": {"value": e2e_value, "unit": "atom-steps/s", "h2d_bytes_per_step": int(hx.nbytes + hv.nbytes),
                     "d2h_bytes_per_step": int(hf.nbytes + he.nbytes)},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "fp64", "kernel": "k_snap_yi<double,8>", "achieved": y_tf, "peak": fp64_peak,
+            "roofline": {"bound": "fp64", "kernel": "k_snap_y<double,8>", "achieved": y_tf, "peak": fp64_peak,
                          "unit": "TFLOP/s", "frac": y_tf / fp64_peak,
                          "peak_source": "measured FP64 FMA rate of this GPU (library probe); "
                                         "MEASURED_PEAKS.json has no FP64 figure",
