@@ -26,6 +26,7 @@
 #include "y_kernels.cuh"
 
 #include <cuda_bf16.h>
+#include <cuda_pipeline.h>
 #include <math.h>
 #include <string.h>
 #include <algorithm>
@@ -378,7 +379,7 @@ k_fit_du(const double4 *__restrict__ prij, long npairs, SnapGeom gp, double2 *__
 // Every dB/dR term is compile-time: triple k = (j1, j2, j) has the terms
 //   Z(j1, j2, j) . dU_j,  Z(j, j2, j1) . dU_j1,  Z(j, j1, j2) . dU_j2
 // with factors 2, 2 (j+1)/(j1+1), 2 (j+1)/(j2+1) (2, 2, 2 with bnorm), so the
-// 55 sums at 2J = 8 stay in registers and the Z offsets are immediates.  The
+// sums stay in registers and the Z offsets are immediates.  The
 // pair's dU is read one row (layer L, column MB) at a time and every term on
 // layer L is applied to that row.  (With the term list read from a table at
 // run time, acc[k] lived in local memory and each term's read-modify-write
@@ -416,31 +417,69 @@ __device__ __forceinline__ double fdb_dot(const double (&dr)[MAMAX + 1], const d
     return s0 + s1;
 }
 
-template <int TJ, int L, int MB, int MAMAX, int ZS, int K>
-__device__ __forceinline__ void fdb_terms(const double (&dr)[MAMAX + 1], const double (&di)[MAMAX + 1],
-                                          const double2 *__restrict__ Zi, double (&acc)[nbispec(TJ)],
-                                          const int bnorm)
+// operations of triple k: the half-plane entries of its three terms' layers
+__host__ __device__ constexpr int fdb_cost(int tj, int k)
 {
-    if constexpr (K < nbispec(TJ)) {
+    const FitTri t = fit_tri(tj, k);
+    const int l[3] = {t.j, t.j1, t.j2};
+    int n = 0;
+    for (int q = 0; q < 3; q++) n += (l[q] + 1) * ((l[q] + 1) / 2) + (l[q] % 2 == 0 ? l[q] / 2 + 1 : 0);
+    return n;
+}
+// The components are cut into FIT_DB_PARTS runs of triples of about equal cost,
+// each summed by warps of its own: with all 55 sums a thread needs 246 registers,
+// and the eight warps of an SM wait for their loads.  512 configurations, 2J = 8
+// (the whole update): 27.8 ms with one part, 25.2 with two at sixteen warps (29.2
+// where the registers leave eight), 26.1 and 28.7 with three and four, whose sums
+// spill.  A row of dU is read by each part that has a term on its layer.
+constexpr int FIT_DB_PARTS = 2;
+// first triple of part q
+__host__ __device__ constexpr int fdb_first(int tj, int q)
+{
+    int all = 0;
+    for (int k = 0; k < nbispec(tj); k++) all += fdb_cost(tj, k);
+    int n = 0, k = 0;
+    while (k < nbispec(tj) && n * FIT_DB_PARTS + fdb_cost(tj, k) * FIT_DB_PARTS / 2 < all * q) n += fdb_cost(tj, k++);
+    return q == FIT_DB_PARTS ? nbispec(tj) : k;
+}
+template <int TJ, int Q> struct FdbPart {
+    static constexpr int k0 = fdb_first(TJ, Q), k1 = fdb_first(TJ, Q + 1);
+};
+template <int TJ, int L, int Q> __host__ __device__ constexpr bool fdb_uses()   // part Q has a term on layer L
+{
+    for (int k = FdbPart<TJ, Q>::k0; k < FdbPart<TJ, Q>::k1; k++) {
+        const FitTri t = fit_tri(TJ, k);
+        if (t.j == L || t.j1 == L || t.j2 == L) return true;
+    }
+    return false;
+}
+
+template <int TJ, int Q, int L, int MB, int MAMAX, int ZS, int K>
+__device__ __forceinline__ void fdb_terms(const double (&dr)[MAMAX + 1], const double (&di)[MAMAX + 1],
+                                          const double2 *__restrict__ Zi,
+                                          double (&acc)[FdbPart<TJ, Q>::k1 - FdbPart<TJ, Q>::k0], const int bnorm)
+{
+    constexpr int K0 = FdbPart<TJ, Q>::k0;
+    if constexpr (K < FdbPart<TJ, Q>::k1) {
         constexpr FitTri t = fit_tri(TJ, K);
-        if constexpr (t.j == L) acc[K] += 2.0 * fdb_dot<TJ, L, MB, MAMAX, ZS, t.j1, t.j2>(dr, di, Zi);
+        if constexpr (t.j == L) acc[K - K0] += 2.0 * fdb_dot<TJ, L, MB, MAMAX, ZS, t.j1, t.j2>(dr, di, Zi);
         if constexpr (t.j1 == L)
-            acc[K] += (bnorm ? 2.0 : 2.0 * (t.j + 1) / (t.j1 + 1.0)) * fdb_dot<TJ, L, MB, MAMAX, ZS, t.j, t.j2>(dr, di, Zi);
+            acc[K - K0] += (bnorm ? 2.0 : 2.0 * (t.j + 1) / (t.j1 + 1.0)) * fdb_dot<TJ, L, MB, MAMAX, ZS, t.j, t.j2>(dr, di, Zi);
         if constexpr (t.j2 == L)
-            acc[K] += (bnorm ? 2.0 : 2.0 * (t.j + 1) / (t.j2 + 1.0)) * fdb_dot<TJ, L, MB, MAMAX, ZS, t.j, t.j1>(dr, di, Zi);
-        fdb_terms<TJ, L, MB, MAMAX, ZS, K + 1>(dr, di, Zi, acc, bnorm);
+            acc[K - K0] += (bnorm ? 2.0 : 2.0 * (t.j + 1) / (t.j2 + 1.0)) * fdb_dot<TJ, L, MB, MAMAX, ZS, t.j, t.j1>(dr, di, Zi);
+        fdb_terms<TJ, Q, L, MB, MAMAX, ZS, K + 1>(dr, di, Zi, acc, bnorm);
     }
 }
 
 // rows MB.. of layer L (and the layers above): dU row in registers (a middle
 // row's right half has no term; its centre counts 1/2), then its terms
-template <int TJ, int L, int MB, int ZS>
+template <int TJ, int Q, int L, int MB, int ZS>
 __device__ __forceinline__ void fdb_rows(const double2 *__restrict__ d, const long stride,
-                                         const double2 *__restrict__ Zi, double (&acc)[nbispec(TJ)],
-                                         const int bnorm)
+                                         const double2 *__restrict__ Zi,
+                                         double (&acc)[FdbPart<TJ, Q>::k1 - FdbPart<TJ, Q>::k0], const int bnorm)
 {
     if constexpr (L <= TJ) {
-        if constexpr (2 * MB <= L) {
+        if constexpr (2 * MB <= L && fdb_uses<TJ, L, Q>()) {
             constexpr int MAMAX = (2 * MB == L) ? MB : L;
             double dr[MAMAX + 1], di[MAMAX + 1];
 #pragma unroll
@@ -450,10 +489,10 @@ __device__ __forceinline__ void fdb_rows(const double2 *__restrict__ d, const lo
                 dr[ma] = w * v.x;
                 di[ma] = w * v.y;
             }
-            fdb_terms<TJ, L, MB, MAMAX, ZS, 0>(dr, di, Zi, acc, bnorm);
-            fdb_rows<TJ, L, MB + 1, ZS>(d, stride, Zi, acc, bnorm);
+            fdb_terms<TJ, Q, L, MB, MAMAX, ZS, FdbPart<TJ, Q>::k0>(dr, di, Zi, acc, bnorm);
+            fdb_rows<TJ, Q, L, MB + 1, ZS>(d, stride, Zi, acc, bnorm);
         } else {
-            fdb_rows<TJ, L + 1, 0, ZS>(d, stride, Zi, acc, bnorm);
+            fdb_rows<TJ, Q, L + 1, 0, ZS>(d, stride, Zi, acc, bnorm);
         }
     }
 }
@@ -464,14 +503,43 @@ __device__ __forceinline__ void fdb_rows(const double2 *__restrict__ d, const lo
 // + dir: a pair-direction's components are contiguous, so the row gathers
 // (k fastest over threads) read them coalesced.  A CTA takes APC adjacent
 // atoms (APC divides 32, so they share a Z tile) and their pairs, 64 threads
-// per atom: the atoms' Z rows (38 KB per atom at 2J = 8) are copied once into
-// shared memory ([entry][atom]), so every pair-direction reads them there.  Read in place from the tile
+// per atom and part: the atoms' Z rows (38 KB per atom at 2J = 8) are copied
+// once into shared memory ([entry][atom], asynchronously: 25.2 -> 24.3 ms, though
+// with half the warps the plain copy was the faster one, 27.9 against 32.0), so
+// every pair-direction reads them there.  Read in place from the tile
 // layout, each entry sat in its own 128-byte line, 512 bytes from the next:
 // an atom's rows touched 2,386 lines, more than L1 holds for the atoms in
 // flight, and the dot products waited on L2.
-constexpr int FIT_DB_TPA = 64;   // threads per atom
+constexpr int FIT_DB_TPA = 64;   // threads per atom and part
+// part `part` of the components, all pair-directions of the CTA's atoms
+template <int TJ, int APC, int Q>
+__device__ __forceinline__ void fdb_parts(const int part, const long q0, const long n3,
+                                          const double2 *__restrict__ dul, const long stride,
+                                          const int2 *__restrict__ pinfo, const int a0, const long p_lo,
+                                          const double2 *__restrict__ Zs, double *__restrict__ dbdr, const int bnorm)
+{
+    if constexpr (Q < FIT_DB_PARTS) {
+        if (part == Q) {
+            for (long i = threadIdx.x % (FIT_DB_TPA * APC); i < n3; i += FIT_DB_TPA * APC) {
+                const long p = q0 + i / 3;
+                const long t = (p - p_lo) * 3 + (i - (i / 3) * 3);
+                const int atom = pinfo[p].x;
+                constexpr int NK = nbispec(TJ), K0 = FdbPart<TJ, Q>::k0, N = FdbPart<TJ, Q>::k1 - K0;
+                double acc[N];
+#pragma unroll
+                for (int k = 0; k < N; k++) acc[k] = 0.0;
+                fdb_rows<TJ, Q, 0, 0, APC>(dul + t, stride, Zs + (atom - a0), acc, bnorm);
+#pragma unroll
+                for (int k = 0; k < N; k++) dbdr[t * NK + K0 + k] = acc[k];
+            }
+            return;
+        }
+        fdb_parts<TJ, APC, Q + 1>(part, q0, n3, dul, stride, pinfo, a0, p_lo, Zs, dbdr, bnorm);
+    }
+}
+
 template <int TJ, int APC>
-__global__ void __launch_bounds__(FIT_DB_TPA * APC)
+__global__ void __launch_bounds__(FIT_DB_TPA * FIT_DB_PARTS * APC, 4 / APC)
 k_fit_dbdr(const double2 *__restrict__ dul, long stride, const int *__restrict__ poff,
            const int2 *__restrict__ pinfo, int a_lo, int a_hi, long p_lo, const FitTables *__restrict__ T,
            const double2 *__restrict__ Z, int tile_lo, double *__restrict__ dbdr)
@@ -483,23 +551,15 @@ k_fit_dbdr(const double2 *__restrict__ dul, long stride, const int *__restrict__
     const int alo = max(a0, a_lo), ahi = min(a0 + APC, a_hi);
     for (int e = threadIdx.x; e < nz * APC; e += blockDim.x) {
         const int k = e / APC, a = a0 + (e - k * APC);
-        if (a >= alo && a < ahi) Zs[e] = Z[((size_t)((a >> 5) - tile_lo) * nz + k) * 32 + (a & 31)];
+        if (a >= alo && a < ahi)
+            __pipeline_memcpy_async(Zs + e, Z + ((size_t)((a >> 5) - tile_lo) * nz + k) * 32 + (a & 31), sizeof(double2));
     }
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
     __syncthreads();
     if (alo >= ahi) return;
     const long q0 = poff[alo], n3 = 3 * (long)(poff[ahi] - q0);
-    for (long i = threadIdx.x; i < n3; i += blockDim.x) {
-        const long p = q0 + i / 3;
-        const long t = (p - p_lo) * 3 + (i - (i / 3) * 3);
-        const int atom = pinfo[p].x;
-        constexpr int NK = nbispec(TJ);
-        double acc[NK];
-#pragma unroll
-        for (int k = 0; k < NK; k++) acc[k] = 0.0;
-        fdb_rows<TJ, 0, 0, APC>(dul + t, stride, Zs + (atom - a0), acc, bnorm);
-#pragma unroll
-        for (int k = 0; k < NK; k++) dbdr[t * NK + k] = acc[k];
-    }
+    fdb_parts<TJ, APC, 0>(threadIdx.x / (FIT_DB_TPA * APC), q0, n3, dul, stride, pinfo, a0, p_lo, Zs, dbdr, bnorm);
 }
 
 // ---------------------------------------------------------------------------
@@ -987,10 +1047,10 @@ static int fit_dbdr_apc(mdp_fit *h, const mdp_fit::Chunk &ck)
     const long nt = 3 * (ck.p_hi - ck.p_lo);
     const size_t sm = (size_t)h->tab.nz * APC * sizeof(double2);
     int per_sm = 0;
-    if (kernel_setup((const void *)k_fit_dbdr<TJ, APC>, FIT_DB_TPA * APC, sm, &per_sm, "k_fit_dbdr")) return -1;
+    if (kernel_setup((const void *)k_fit_dbdr<TJ, APC>, FIT_DB_TPA * FIT_DB_PARTS * APC, sm, &per_sm, "k_fit_dbdr")) return -1;
     const int a0 = ck.a_lo & ~(APC - 1);
     const unsigned g = (unsigned)((ck.a_hi - a0 + APC - 1) / APC);
-    k_fit_dbdr<TJ, APC><<<g, FIT_DB_TPA * APC, sm, h->s>>>(
+    k_fit_dbdr<TJ, APC><<<g, FIT_DB_TPA * FIT_DB_PARTS * APC, sm, h->s>>>(
         h->dul.as<double2>(), nt, h->poff.as<int>(), h->fp.pinfo.as<int2>(), ck.a_lo, ck.a_hi, ck.p_lo,
         h->tabs.as<FitTables>(), h->Z.as<double2>(), ck.t_lo, h->dbdr.as<double>());
     return 0;
