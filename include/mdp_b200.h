@@ -60,6 +60,11 @@ int mdp_snap_ncoeff(int twojmax);
  *   neighlist inum x neighmax rows, neighnum[inum]
  *   eatom    inum, fatom inum x 3 AoS, vatom 6 x inum SoA (may be NULL)
  * Outputs are overwritten (the reference accumulates into zeroed arrays).
+ * The call queues its work on cuda_stream and returns.  Calls from any thread
+ * and on any stream of a device are safe: they share that device's work
+ * buffers and run one after the other there.  A call captured into a graph uses
+ * the same buffers at every replay, so a replay must not overlap other calls,
+ * and none may grow them (by more atoms or rows) while the graph is in use.
  * ------------------------------------------------------------------------- */
 int mdp_snap_compute_device(const mdp_snap_params *p, int precision, const double *x, const int *alist,
                             const int *neighlist, const int *neighnum, int inum, int anum, int neighmax,

@@ -12,6 +12,7 @@
 #include <stdlib.h>
 #include <string.h>
 #include <algorithm>
+#include <map>
 #include <mutex>
 
 namespace mdp {
@@ -583,9 +584,51 @@ struct OneShot {
     SnapModel model;
     Neighbors nb;
     ForcePath fp;
-    DevBuf x4, f4, xin, alist_tmp, types;
+    DevBuf x4, f4, xin, types;
+    cudaEvent_t done = nullptr;   // behind the last call's work on these buffers
 };
 static std::mutex g_os_mu;
+
+// The buffers of the current device, for one kind of call.  Held for the process's
+// life; callers hold g_os_mu.
+static int one_shot(std::map<int, OneShot> &kind, OneShot **os)
+{
+    int dev = 0;
+    MDP_CUDA_TRY(cudaGetDevice(&dev));
+    *os = &kind[dev];
+    return 0;
+}
+
+// Calls on several streams take turns on a device's buffers: a call's work is
+// queued behind that of the call before, whichever stream that was on.  (A handle
+// tells nothing: streams come and go at one address, and the per-thread default
+// stream has one handle for all threads.)  While its stream is being captured a
+// call can neither wait for work outside the graph nor be waited for.
+class OneShotTurn {
+public:
+    OneShotTurn(OneShot &os, cudaStream_t s) : os_(os), s_(s) {}
+    OneShotTurn(const OneShotTurn &) = delete;
+    OneShotTurn &operator=(const OneShotTurn &) = delete;
+    int begin()
+    {
+        cudaStreamCaptureStatus st;
+        MDP_CUDA_TRY(cudaStreamIsCapturing(s_, &st));
+        if (st != cudaStreamCaptureStatusNone) return 0;
+        if (!os_.done) MDP_CUDA_TRY(cudaEventCreateWithFlags(&os_.done, cudaEventDisableTiming));
+        MDP_CUDA_TRY(cudaStreamWaitEvent(s_, os_.done, 0));   // an event not yet recorded holds nothing up
+        on_ = true;
+        return 0;
+    }
+    ~OneShotTurn()   // also behind the part of a call that was queued before an error
+    {
+        if (on_) cudaEventRecord(os_.done, s_);
+    }
+
+private:
+    OneShot &os_;
+    cudaStream_t s_;
+    bool on_ = false;
+};
 
 // types 1..ne on the host; 0 or -1 with the error set
 static int check_types(const int *t, long n, int ne)
@@ -605,9 +648,10 @@ static int compute_host(const mdp_snap_params *p, int precision, int natoms, con
 {
     std::lock_guard<std::mutex> lk(g_os_mu);
     if (!x || !box || natoms <= 0) { set_error("bad arguments"); return -1; }
-    static OneShot os;
-    int dev = 0;
-    MDP_CUDA_TRY(cudaGetDevice(&dev));
+    static std::map<int, OneShot> kind;
+    OneShot *mine;
+    if (one_shot(kind, &mine)) return -1;
+    OneShot &os = *mine;   // (all work below is on the default stream)
     if (model_init(os.model, p)) return -1;
     const int *types_dev = nullptr;
     if (os.model.ne > 1) {
@@ -687,10 +731,11 @@ static int compute_device(const mdp_snap_params *p, int precision, const double 
                           int neighmax, double *eatom, double *fatom, double *vatom, void *stream)
 {
     std::lock_guard<std::mutex> lk(g_os_mu);
-    static OneShot os;
+    static std::map<int, OneShot> kind;
+    OneShot *mine;
+    if (one_shot(kind, &mine)) return -1;
+    OneShot &os = *mine;
     cudaStream_t s = (cudaStream_t)stream;
-    int dev = 0;
-    MDP_CUDA_TRY(cudaGetDevice(&dev));
     if (model_init(os.model, p)) return -1;
     if (os.model.ne > 1) {
         if (!atomtype) { set_error("a model with %d element types needs the atom types", os.model.ne); return -1; }
@@ -704,8 +749,10 @@ static int compute_device(const mdp_snap_params *p, int precision, const double 
         os.nb.cursor.ensure(sizeof(int) * inum) || os.nb.rlist.ensure(sizeof(long long) * (size_t)inum * neighmax) ||
         os.nb.scan_tmp.ensure(sizeof(int) * scan_tmp_ints(inum)))
         return -1;
+    OneShotTurn turn(os, s);
+    if (turn.begin()) return -1;
     k_aos_to_d4<<<(anum + 255) / 256, 256, 0, s>>>(x, os.x4.as<double4>(), anum);
-    const int tb = 256, gb = (inum + tb - 1) / tb;
+    const int tb = 256;
     MDP_CUDA_TRY(cudaMemsetAsync(os.nb.rcount.p, 0, sizeof(int) * inum, s));
     const unsigned gs = (unsigned)(((long)inum * neighmax + tb - 1) / tb);   // one thread per slot
     if (gs) k_rev_count<<<gs, tb, 0, s>>>(neighlist, neighnum, alist, inum, neighmax, os.nb.rcount.as<int>());
