@@ -754,12 +754,12 @@ static int compute_device(const mdp_snap_params *p, int precision, const double 
     k_aos_to_d4<<<(anum + 255) / 256, 256, 0, s>>>(x, os.x4.as<double4>(), anum);
     const int tb = 256;
     MDP_CUDA_TRY(cudaMemsetAsync(os.nb.rcount.p, 0, sizeof(int) * inum, s));
-    const unsigned gs = (unsigned)(((long)inum * neighmax + tb - 1) / tb);   // one thread per slot
-    if (gs) k_rev_count<<<gs, tb, 0, s>>>(neighlist, neighnum, alist, inum, neighmax, os.nb.rcount.as<int>());
+    const unsigned gw = (unsigned)(((long)inum * 32 + tb - 1) / tb);   // one warp per row
+    k_rev_count<<<gw, tb, 0, s>>>(neighlist, neighnum, alist, inum, neighmax, os.nb.rcount.as<int>());
     if (exclusive_scan(os.nb.rcount.as<int>(), os.nb.roff.as<int>(), inum, os.nb.scan_tmp.as<int>(), s)) return -1;
     MDP_CUDA_TRY(cudaMemsetAsync(os.nb.cursor.p, 0, sizeof(int) * inum, s));
-    if (gs) k_rev_fill<<<gs, tb, 0, s>>>(neighlist, neighnum, alist, inum, neighmax, os.nb.roff.as<int>(),
-                                         os.nb.cursor.as<int>(), os.nb.rlist.as<long long>());
+    k_rev_fill<<<gw, tb, 0, s>>>(neighlist, neighnum, alist, inum, neighmax, os.nb.roff.as<int>(),
+                                 os.nb.cursor.as<int>(), os.nb.rlist.as<long long>());
     k_rev_sort<<<std::min((inum + 7) / 8, num_sms() * 8), 256, 0, s>>>(inum, os.nb.roff.as<int>(), os.nb.rlist.as<long long>());
     if (force_compute(os.fp, os.model, precision, os.x4.as<double4>(), inum, neighlist, neighnum, neighmax,
                       (long)inum * neighmax, os.nb.roff.as<int>(), os.nb.rlist.as<long long>(), eatom,

@@ -280,30 +280,32 @@ k_neigh_build(const double4 *__restrict__ x, int inum, const __grid_constant__ B
 
 // reverse index: for each owner o, the (i, slot) entries whose neighbour is
 // an image of o; used to gather -dE onto owners without atomics
-// One thread per slot of the rows.
-__device__ __forceinline__ long slot_row(const long t, const int nm)
-{
-    return t <= 0xffffffffL ? (long)((unsigned)t / (unsigned)nm) : t / nm;   // 32-bit division where it serves
-}
-
+// One warp per row, its lanes striding over the entries, so that the work goes
+// with the entries and not with the rows' capacity: with a thread per slot, rows
+// of 1,000 slots made a call of 128,000 atoms (2J = 4) take 1.63 ms, against
+// 1.04 here and 1.05 at 64 slots in either form.
 __global__ void k_rev_count(const int *__restrict__ nlist, const int *__restrict__ nnum, const int *__restrict__ alist,
                             int inum, int nm, int *__restrict__ rcount)
 {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long i = slot_row(t, nm);
-    if (i >= inum || (int)(t - i * nm) >= nnum[i]) return;
-    atomicAdd(&rcount[alist[nlist[t]]], 1);
+    const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (i >= inum) return;
+    const int n = min(nnum[i], nm);
+    const int *row = nlist + i * nm;
+    for (int l = threadIdx.x & 31; l < n; l += 32) atomicAdd(&rcount[alist[row[l]]], 1);
 }
 
 __global__ void k_rev_fill(const int *__restrict__ nlist, const int *__restrict__ nnum, const int *__restrict__ alist,
                            int inum, int nm, const int *__restrict__ roff, int *__restrict__ cursor,
                            long long *__restrict__ rlist)
 {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long i = slot_row(t, nm);
-    if (i >= inum || (int)(t - i * nm) >= nnum[i]) return;
-    const int o = alist[nlist[t]];
-    rlist[roff[o] + atomicAdd(&cursor[o], 1)] = t;
+    const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (i >= inum) return;
+    const int n = min(nnum[i], nm);
+    const int *row = nlist + i * nm;
+    for (int l = threadIdx.x & 31; l < n; l += 32) {
+        const int o = alist[row[l]];
+        rlist[roff[o] + atomicAdd(&cursor[o], 1)] = (long long)i * nm + l;
+    }
 }
 
 // Each owner's reverse entries ascending, so the tally sums in a fixed order.

@@ -588,13 +588,13 @@ int neighbor_build(Neighbors &nb, const BoxParams &bp, double4 *x, int inum, dou
         x, inum, bp, nb.cidx.as<int>(), nb.cstart.as<int>(), nb.catoms.as<int>(), rc * rc, nm, nb.nlist.as<int>(),
         nb.nnum.as<int>(), nb.status.as<int>());
     MDP_CUDA_TRY(cudaMemsetAsync(nb.rcount.p, 0, sizeof(int) * inum, s));
-    const unsigned gs = (unsigned)(((long)inum * nm + tb - 1) / tb);   // one thread per slot
-    if (gs) k_rev_count<<<gs, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum, nm,
-                                          nb.rcount.as<int>());
+    const unsigned gw = (unsigned)(((long)inum * 32 + tb - 1) / tb);   // one warp per row
+    k_rev_count<<<gw, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum, nm,
+                                  nb.rcount.as<int>());
     if (exclusive_scan(nb.rcount.as<int>(), nb.roff.as<int>(), inum, tmp, s)) return -1;
     MDP_CUDA_TRY(cudaMemsetAsync(nb.cursor.p, 0, sizeof(int) * inum, s));
-    if (gs) k_rev_fill<<<gs, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum, nm,
-                                         nb.roff.as<int>(), nb.cursor.as<int>(), nb.rlist.as<long long>());
+    k_rev_fill<<<gw, tb, 0, s>>>(nb.nlist.as<int>(), nb.nnum.as<int>(), nb.alist.as<int>(), inum, nm,
+                                 nb.roff.as<int>(), nb.cursor.as<int>(), nb.rlist.as<long long>());
     k_rev_sort<<<std::min((inum + 7) / 8, num_sms() * 8), 256, 0, s>>>(inum, nb.roff.as<int>(), nb.rlist.as<long long>());
     count_launches(8);
     int hs[2] = {0, 0};
