@@ -37,10 +37,17 @@ namespace mdp {
 // ---------------------------------------------------------------------------
 // pairs: every atom against every atom of its configuration and the 27 images
 // ---------------------------------------------------------------------------
-// One warp per atom: the lanes test 32 (atom, image) candidates at a time in the
-// list's order, a ballot ranks the pairs found, and their geometry is evaluated
-// 32 pairs at a time.  (A thread per atom walks some 27 x 150 candidates one
-// after the other: 0.17 + 0.89 ms for 2,700 atoms.)
+// One warp per atom.  A lane takes one atom of the configuration and its 27
+// images, so that the other atom is read once and the shifts, which a warp forms
+// once, are the same for all lanes; the images found are bits of a mask.  Pairs
+// are listed by atom, then image: a scan over the lanes ranks them, and their
+// geometry is evaluated 32 pairs at a time.  The FP64 pipe bounds it (eleven
+// instructions a candidate) where the batch is large.  With a lane per candidate,
+// each taking its atom and shift apart from the candidate's number, setting a
+// batch of 4,096 configurations took 95 ms (58 here, mostly host work), and 20
+// cells of 2,048 atoms 13.0 ms (4.4 here).  A thread per atom took 76 and 12.2,
+// but walks some 27 x 150 candidates one after the other when the batch is small:
+// 0.17 + 0.89 ms for 2,700 atoms.
 constexpr int FIT_PAIR_WARPS = 4;
 template <bool EMIT>
 __global__ void __launch_bounds__(FIT_PAIR_WARPS * 32)
@@ -49,66 +56,81 @@ k_fit_pairs(const double4 *__restrict__ x, const int *__restrict__ cfg, const in
             int *__restrict__ pcount, const int *__restrict__ poff, double4 *__restrict__ prij,
             double4 *__restrict__ pab, int2 *__restrict__ pinfo)
 {
-    __shared__ int found[FIT_PAIR_WARPS][64];   // candidates of pairs not yet emitted
+    __shared__ double shifts[FIT_PAIR_WARPS][27][3];
+    __shared__ int queues[EMIT ? FIT_PAIR_WARPS : 1][32 + 32 * 27];   // 27 atom + image of pairs not yet emitted
     const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
     const int i = blockIdx.x * FIT_PAIR_WARPS + wb;
     if (i >= natoms) return;   // whole warps leave together
     const int c = cfg[i], a0 = ca0[c], n = cn[c];
-    // lattice vectors a, b, c of the configuration's cell (rows of cbox)
-    const double4 la = cbox[3 * c], lb = cbox[3 * c + 1], lc = cbox[3 * c + 2], xi = x[i];
-    auto vec = [&](const int q, double &d0, double &d1, double &d2) {
-        const int jj = q / 27, im = q - 27 * jj;
-        const double4 xj = x[a0 + jj];
-        const double u = im % 3 - 1, v = (im / 3) % 3 - 1, w = im / 9 - 1;
-        const double sx = u * la.x + v * lb.x + w * lc.x, sy = u * la.y + v * lb.y + w * lc.y,
-                     sz = u * la.z + v * lb.z + w * lc.z;
-        d0 = xj.x + sx - xi.x;
-        d1 = xj.y + sy - xi.y;
-        d2 = xj.z + sz - xi.z;
-    };
-    int cnt = 0, p = EMIT ? poff[i] : 0, nf = 0;
-    auto emit = [&](const int m) {   // the first m <= 32 candidates of found
+    double(*const sh)[3] = shifts[wb];
+    if (lane < 27) {
+        // lattice vectors a, b, c of the configuration's cell (rows of cbox)
+        const double4 la = cbox[3 * c], lb = cbox[3 * c + 1], lc = cbox[3 * c + 2];
+        const double u = lane % 3 - 1, v = (lane / 3) % 3 - 1, w = lane / 9 - 1;
+        sh[lane][0] = u * la.x + v * lb.x + w * lc.x;
+        sh[lane][1] = u * la.y + v * lb.y + w * lc.y;
+        sh[lane][2] = u * la.z + v * lb.z + w * lc.z;
+    }
+    __syncwarp();
+    const double4 xi = x[i];
+    int cnt = 0, p = 0, nf = 0;
+    int *const found = queues[EMIT ? wb : 0];
+    if constexpr (EMIT) p = poff[i];
+    auto emit = [&](const int f, const int m) {   // the m <= 32 pairs from found[f] on
         if (lane < m) {
-            const int q = found[wb][lane];
-            double d0, d1, d2;
-            vec(q, d0, d1, d2);
+            const int q = found[f + lane], jj = q / 27, im = q - 27 * jj;
+            const double4 xj = x[a0 + jj];
+            const double d0 = xj.x + sh[im][0] - xi.x, d1 = xj.y + sh[im][1] - xi.y, d2 = xj.z + sh[im][2] - xi.z;
             PairGeo g;
             pair_geometry<false>(g, d0, d1, d2, gp);
             prij[p + lane] = make_double4(d0, d1, d2, g.sfac);
             pab[p + lane] = make_double4(g.ar, g.ai, g.br, g.bi);
-            pinfo[p + lane] = make_int2(i, a0 + q / 27);
+            pinfo[p + lane] = make_int2(i, a0 + jj);
         }
         p += m;
     };
-    for (int q0 = 0; q0 < 27 * n; q0 += 32) {
-        const int q = q0 + lane;
-        bool pair = false;
-        if (q < 27 * n) {
-            double d0, d1, d2;
-            vec(q, d0, d1, d2);
+    for (int j0 = 0; j0 < n; j0 += 32) {
+        const int jj = j0 + lane;
+        const double4 xj = x[a0 + min(jj, n - 1)];
+        unsigned mask = 0;
+#pragma unroll 9
+        for (int im = 0; im < 27; im++) {
+            const double d0 = xj.x + sh[im][0] - xi.x, d1 = xj.y + sh[im][1] - xi.y, d2 = xj.z + sh[im][2] - xi.z;
             const double rsq = d0 * d0 + d1 * d1 + d2 * d2;
-            pair = rsq < gp.rcutsq && rsq > 1e-20;
+            if (rsq < gp.rcutsq && rsq > 1e-20) mask |= 1u << im;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, pair);
+        if (jj >= n) mask = 0;
         if constexpr (EMIT) {
-            if (pair) found[wb][nf + __popc(m & ((1u << lane) - 1u))] = q;
-            nf += __popc(m);
-            __syncwarp();
-            if (nf >= 32) {
-                emit(32);
-                __syncwarp();
-                nf -= 32;
-                const int v = found[wb][32 + lane];
-                __syncwarp();
-                if (lane < nf) found[wb][lane] = v;
-                __syncwarp();
+            const int k = __popc(mask);
+            int off = k;   // inclusive sum over the lanes
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, off, o);
+                if (lane >= o) off += t;
             }
+            const int total = __shfl_sync(0xffffffffu, off, 31);
+            for (int *to = found + nf + off - k; mask; mask &= mask - 1) *to++ = 27 * jj + __ffs(mask) - 1;
+            __syncwarp();
+            nf += total;   // at most 31 + 32 * 27
+            int f = 0;
+            for (; nf - f >= 32; f += 32) emit(f, 32);
+            nf -= f;
+            if (f) {
+                const int v = lane < nf ? found[f + lane] : 0;
+                __syncwarp();
+                if (lane < nf) found[lane] = v;
+            }
+            __syncwarp();
         } else {
-            cnt += __popc(m);
+            cnt += __popc(mask);
         }
     }
-    if constexpr (EMIT) emit(nf);
-    else if (lane == 0) pcount[i] = cnt;
+    if constexpr (EMIT) {
+        emit(0, nf);
+    } else {
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0) pcount[i] = cnt;
+    }
 }
 
 // ZBL reference potential of every atom of the batch (the pair term that MDP's
