@@ -292,7 +292,7 @@ static int run_yi(RefCtx &c, int inum, int tj, cudaStream_t s)
 {
     const long ntiles = (inum + 31) / 32;
     if (c.fp.Y.ensure(sizeof(double2) * ntiles * 32 * yh_count(tj)) || c.etmp.ensure(sizeof(double) * inum)) return -1;
-    return launch_yi_full(tj, c.model.yd, c.fp, inum, c.etmp.as<double>(), nullptr, s);
+    return launch_yi_full(tj, c.model.yd, c.model.yl, c.fp, inum, c.etmp.as<double>(), nullptr, s);
 }
 
 int ref_snap_ui(double *ur, double *ui, const double *rij, double rcut, double wj, double rfac0, double rmin0,
@@ -317,9 +317,9 @@ int ref_snap_ui(double *ur, double *ui, const double *rij, double rcut, double w
     {                                                                                                              \
         const size_t sm = (size_t)UI_WARPS * (idxu_count(TJ) + 32 * (TJ + 1)) * sizeof(double2);                  \
         int per_sm = 0;                                                                                            \
-        if (kernel_setup((const void *)k_snap_ui<double, TJ>, UI_WARPS * 32, sm, &per_sm, "k_snap_ui"))            \
+        if (kernel_setup((const void *)k_snap_ui<TJ>, UI_WARPS * 32, sm, &per_sm, "k_snap_ui"))            \
             return -1;                                                                                             \
-        k_snap_ui<double, TJ><<<blocks, UI_WARPS * 32, sm, s>>>(c.off.as<int>(), c.fp.prij.as<double4>(),          \
+        k_snap_ui<TJ><<<blocks, UI_WARPS * 32, sm, s>>>(c.off.as<int>(), c.fp.prij.as<double4>(),          \
                                                                 inum, c.model.geom, ur, ui);                       \
     }
     switch (tj) {
@@ -378,7 +378,7 @@ int ref_snap_yi_beta(double *yr, double *yi, const double *ur, const double *ui,
     if (load_tiles(c, ur, ui, inum, tj, s)) return -1;
     const long ntiles = (inum + 31) / 32;
     if (c.fp.Y.ensure(sizeof(double2) * ntiles * 32 * yh_count(tj))) return -1;
-    if (launch_yi_full(tj, c.model.yd, c.fp, inum, nullptr, beta, s)) return -1;
+    if (launch_yi_full(tj, c.model.yd, c.model.yl, c.fp, inum, nullptr, beta, s)) return -1;
     const long n = (long)inum * idxu_count(tj);
     k_ytiles_to_ref<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(c.fp.Y.as<double2>(), inum, tj, yh_count(tj), yr, yi);
     MDP_CUDA_TRY(cudaGetLastError());
@@ -604,9 +604,9 @@ int ref_snap_ui_me(double *ur, double *ui, const double *rij, const double *rade
     {                                                                                                              \
         const size_t sm = (size_t)UI_WARPS * (idxu_count(TJ) + 32 * (TJ + 1)) * sizeof(double2);                  \
         int per_sm = 0;                                                                                            \
-        if (kernel_setup((const void *)k_snap_ui<double, TJ>, UI_WARPS * 32, sm, &per_sm, "k_snap_ui"))            \
+        if (kernel_setup((const void *)k_snap_ui<TJ>, UI_WARPS * 32, sm, &per_sm, "k_snap_ui"))            \
             return -1;                                                                                             \
-        k_snap_ui<double, TJ><<<blocks, UI_WARPS * 32, sm, s>>>(c.off.as<int>(), c.fp.prij.as<double4>(),          \
+        k_snap_ui<TJ><<<blocks, UI_WARPS * 32, sm, s>>>(c.off.as<int>(), c.fp.prij.as<double4>(),          \
                                                                 (int)nv, c.model.geom, ur, ui,                     \
                                                                 c.fp.pcw.as<double2>(), inum);                     \
     }
@@ -700,10 +700,10 @@ int ref_snap_yi_me(double *yr, double *yi, const double *ur, const double *ui, c
 #define MDP_YI_ME(TJ)                                                                                              \
     {                                                                                                              \
         const size_t sm = yi_me_smem_bytes<TJ>();                                                                  \
-        if (kernel_setup((const void *)k_snap_yi_me<TJ>, YI_WARPS * 32, sm, &per_sm, "k_snap_yi_me")) \
+        if (kernel_setup((const void *)k_snap_yi_me<TJ>, YI_WARPS * 32, sm, &per_sm, "k_snap_yi_me"))          \
             return -1;                                                                                             \
-        k_snap_yi_me<TJ><<<std::min(A.ntiles, num_sms() * per_sm), YI_WARPS * 32, sm, s>>>(          \
-            Ut, inum, c.model.yd, A, Y);                                                                           \
+        k_snap_yi_me<TJ><<<std::min(A.ntiles, num_sms() * per_sm), YI_WARPS * 32, sm, s>>>(                       \
+            Ut, inum, c.model.yd, c.model.yl, A, Y);                                                               \
     }
     switch (tj) {
     case 4: MDP_YI_ME(4) break;

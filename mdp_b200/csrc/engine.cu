@@ -720,12 +720,6 @@ int mdp_snap_compute_host_typed(const mdp_snap_params *p, int precision, int nat
                         neighnum, anum_out, alist_out, xall_out, alist_cap);
 }
 
-__global__ void k_copy_int(const int *__restrict__ a, int *__restrict__ b, long n)
-{
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = a[i];
-}
-
 static int compute_device(const mdp_snap_params *p, int precision, const double *x, const int *atomtype,
                           const int *alist, const int *neighlist, const int *neighnum, int inum, int anum,
                           int neighmax, double *eatom, double *fatom, double *vatom, void *stream)

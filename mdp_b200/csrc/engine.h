@@ -108,6 +108,7 @@ struct SnapModel {
     SnapGeom geom;
     YParams<double> yd;
     YParams<float> yf;
+    YiLayout yl;          // stage entry points: warps of k_snap_yi
     YParams<double> yq;   // quadratic: unit coefficients (multiplicities only), per-atom coefficients from B
     QuadParams quad;
     int nu, nyh, ncoeff;
@@ -137,7 +138,6 @@ struct ForcePath {
     const int *u_welem = nullptr;     // U stage: element of each atom, for wself per element block
     int u_ipad = 0;
     const double2 *fr_pcw = nullptr;  // dE/dr stage: per-pair cutoff / weight
-    int natoms_cap = 0, nm_cap = 0;
     // per-stage timing (CUDA events on the launching stream), enabled on demand
     bool timing = false;
     cudaEvent_t ev[8] = {};
@@ -152,8 +152,8 @@ template <typename T, int TJ>
 int launch_yi(const YParams<T> &yp, ForcePath &fp, int inum, double *eatom, cudaStream_t s);
 template <int TJ>
 int launch_yi_pa_d(const YParams<double> &yp, ForcePath &fp, int inum, const double *G, cudaStream_t s);
-int launch_yi_full(int tj, const YParams<double> &yp, ForcePath &fp, int inum, double *eatom, const double *G,
-                   cudaStream_t s);
+int launch_yi_full(int tj, const YParams<double> &yp, const YiLayout &yl, ForcePath &fp, int inum, double *eatom,
+                   const double *G, cudaStream_t s);
 // bispectrum of fp.Ut, bout[k * inum + atom]
 template <typename T, int TJ>
 int launch_b(const ForcePath &fp, int inum, int bnorm, int bzero, double *bout, cudaStream_t s);

@@ -66,7 +66,7 @@ template <typename T, int TJ> constexpr size_t fc_smem_bytes()
 {
     return (size_t)fc_most<TJ>() * 3 * fc_cap<T>() * sizeof(typename cplx<T>::type) +
            fc_pairs<T>() * (4 * sizeof(double) + 4 * sizeof(T) + sizeof(int)) +
-           fc_base<TJ>(FcJobs<TJ>::n) * sizeof(FcEntry) + sizeof(int) * 2;
+           fc_base<TJ>(FcJobs<TJ>::n) * sizeof(FcEntry) + sizeof(int);
 }
 
 // Y tile offsets and factors of entry m of row (J, mb)
@@ -236,12 +236,12 @@ k_snap_fc(const double4 *__restrict__ prij, const double4 *__restrict__ pab, con
     FcEntry *ent = reinterpret_cast<FcEntry *>(Cs + fc_most<TJ>() * 3 * CAP);
     T *sab = reinterpret_cast<T *>(ent + fc_base<TJ>(FcJobs<TJ>::n));       // [a, b][pair]
     int *satom = reinterpret_cast<int *>(sab + 4 * NP);                     // [pair]
-    int *anext = satom + NP;                                                // first atom of this and the next turn
+    int *afirst = satom + NP;                                               // the window's first atom
     fc_entries<TJ, 0>(ent, threadIdx.x, FC_THREADS);
     const int npairs = *pnum;
     // windows of NP consecutive pairs (the loop bounds are uniform over the CTA)
     for (int base = blockIdx.x * NP; base < npairs; base += gridDim.x * NP) {
-        if (threadIdx.x < 2) anext[threadIdx.x] = INT_MAX;
+        if (threadIdx.x == 0) *afirst = INT_MAX;
         __syncthreads();
         for (int q = threadIdx.x; q < NP; q += FC_THREADS) {
             const int p = base + q;
@@ -256,10 +256,10 @@ k_snap_fc(const double4 *__restrict__ prij, const double4 *__restrict__ pab, con
             }
             satom[q] = atom;
             const int first = __reduce_min_sync(0xffffffffu, atom);
-            if ((threadIdx.x & 31) == 0) atomicMin(&anext[0], first);
+            if ((threadIdx.x & 31) == 0) atomicMin(afirst, first);
         }
         __syncthreads();
-        int a0 = anext[0], turn = 0;
+        int a0 = *afirst;
         while (a0 != INT_MAX) {
             // the turn's last atom, and the first one of the next turn
             int last = a0, after = INT_MAX;
@@ -272,7 +272,6 @@ k_snap_fc(const double4 *__restrict__ prij, const double4 *__restrict__ pab, con
             after = __reduce_min_sync(0xffffffffu, after);
             fc_job<T, TJ, 0>(a0, na, Y, ent, Cs, sums, sab, satom);
             a0 = after;
-            turn++;
         }
         // a thread's pairs are the ones it has summed
         for (int q = threadIdx.x; q < NP; q += FC_THREADS) {

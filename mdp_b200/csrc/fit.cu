@@ -268,7 +268,7 @@ k_fit_zbt(const double2 *__restrict__ Ut, int natoms, const FitTables *__restric
         for (int k = w; k < T->ntri; k += zb_warps<TJ>()) {
             const FitTriple tr = T->tr[k];
             const int j = tr.j;
-            const FitCoupling cp = T->cp[tr.coup[0]];
+            const FitCoupling cp = T->cp[tr.coup];
             double s = 0.0;
             for (int mb = 0; 2 * mb <= j; mb++)
                 for (int ma = 0; ma <= j; ma++) {
@@ -929,26 +929,8 @@ static void fit_tables(FitTables &T, int tj, int bnorm, int bzero)
             for (int j = j1 - j2; j <= std::min(tj, j1 + j2); j += 2) {
                 if (j < j1) continue;
                 FitTriple &t = T.tr[T.ntri++];
-                t.j1 = j1; t.j2 = j2; t.j = j;
-                // cpuComputeDbidrj:826-1013: z(j1,j2,j) with dU_j; z(j,j2,j1) with dU_j1
-                // times (j+1)/(j1+1); z(j,j1,j2) with dU_j2 times (j+1)/(j2+1)
-                t.layer[0] = j; t.coup[0] = idx[j1][j2][j]; t.fac[0] = 1.0;
-                t.layer[1] = j1; t.coup[1] = idx[j][j2][j1]; t.fac[1] = bnorm ? 1.0 : (j + 1) / (j1 + 1.0);
-                t.layer[2] = j2; t.coup[2] = idx[j][j1][j2]; t.fac[2] = bnorm ? 1.0 : (j + 1) / (j2 + 1.0);
+                t.j1 = j1; t.j2 = j2; t.j = j; t.coup = idx[j1][j2][j];
             }
-    int q = 0;
-    for (int L = 0; L < JD; L++) {
-        T.lt_off[L] = q;
-        for (int k = 0; k < T.ntri; k++)
-            for (int r = 0; r < 3; r++)
-                if (T.tr[k].layer[r] == L) {
-                    T.lt_k[q] = k;
-                    T.lt_z[q] = T.cp[T.tr[k].coup[r]].zoff;
-                    T.lt_fac[q] = 2.0 * T.tr[k].fac[r];
-                    q++;
-                }
-        T.lt_n[L] = q - T.lt_off[L];
-    }
 }
 
 }  // namespace mdp

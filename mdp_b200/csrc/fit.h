@@ -16,18 +16,12 @@ struct FitCoupling {
     int j1, j2, j, zoff;          // Z rows of this coupling start at zoff (per atom)
 };
 struct FitTriple {
-    int j1, j2, j;
-    int layer[3], coup[3];        // the three dB/dR terms: dU layer and Z coupling
-    double fac[3];
+    int j1, j2, j, coup;          // coup: coupling (j1, j2, j)
 };
 struct FitTables {
     int ncoup, ntri, nz, tj, bnorm, bzero;
     FitCoupling cp[FIT_NCP];
     FitTriple tr[FIT_NT];
-    // the dB/dR terms grouped by their dU layer: lt_off[L] .. lt_off[L] + lt_n[L]
-    int lt_n[JD], lt_off[JD];
-    int lt_k[3 * FIT_NT], lt_z[3 * FIT_NT];
-    double lt_fac[3 * FIT_NT];
 };
 
 }  // namespace mdp

@@ -249,61 +249,47 @@ int model_init(SnapModel &m, const mdp_snap_params *p)
     m.yd.e0 = e0;
     m.yf.e0 = e0;
 
-    // Y-kernel warp assignment per output layer j: rows mb get warps in
-    // proportion to their cost (sum over couplings of items x terms per item);
-    // a row with k warps is split by row-pair index ib modulo k
-    auto assign = [&](int nw, unsigned char (*lmb)[YI_MAXW], unsigned char (*lo)[YI_MAXW],
-                      unsigned char (*lst)[YI_MAXW]) {
-        for (int j = 0; j < JD; j++)
-            for (int w = 0; w < YI_MAXW; w++) { lmb[j][w] = 255; lo[j][w] = 0; lst[j][w] = 1; }
-        for (int j = 0; j <= tj; j++) {
-            const int R = j / 2 + 1;
-            std::vector<double> cost(R, 0.0);
-            for (int mb = 0; mb < R; mb++)
-                for (int j1 = 0; j1 <= tj; j1++)
-                    for (int j2 = 0; j2 <= j1; j2++) {
-                        if (!coupling_ok(j1, j2, j)) continue;
-                        int terms = 0;
-                        for (int ma = 0; ma <= j; ma++) {
-                            int ma1min = std::max(0, (2 * ma - j - j2 + j1) / 2);
-                            terms += std::min(j1, (2 * ma - j + j2 + j1) / 2) - ma1min + 1;
-                        }
-                        cost[mb] += (double)nb_of(j1, j2, j, mb) * (terms + j1 + j2 + 2);
+    // warps of k_snap_yi per output layer j: rows mb get warps in proportion to
+    // their cost (sum over couplings of items x terms per item); a row with k
+    // warps is split by row-pair index ib modulo k
+    for (int j = 0; j < JD; j++)
+        for (int w = 0; w < YI_WARPS; w++) { m.yl.mb[j][w] = 255; m.yl.o[j][w] = 0; m.yl.st[j][w] = 1; }
+    for (int j = 0; j <= tj; j++) {
+        const int R = j / 2 + 1;
+        std::vector<double> cost(R, 0.0);
+        for (int mb = 0; mb < R; mb++)
+            for (int j1 = 0; j1 <= tj; j1++)
+                for (int j2 = 0; j2 <= j1; j2++) {
+                    if (!coupling_ok(j1, j2, j)) continue;
+                    int terms = 0;
+                    for (int ma = 0; ma <= j; ma++) {
+                        int ma1min = std::max(0, (2 * ma - j - j2 + j1) / 2);
+                        terms += std::min(j1, (2 * ma - j + j2 + j1) / 2) - ma1min + 1;
                     }
-            std::vector<int> nw_row(R, 1);
-            int used = std::min(R, nw);
-            if (R > nw) return -1;
-            while (used < nw) {
-                int best = 0;
-                for (int r = 1; r < R; r++)
-                    if (cost[r] / nw_row[r] > cost[best] / nw_row[best]) best = r;
-                // splitting a row beyond its largest item count buys nothing
-                int maxnb = 0;
-                for (int j1 = 0; j1 <= tj; j1++)
-                    for (int j2 = 0; j2 <= j1; j2++)
-                        if (coupling_ok(j1, j2, j)) maxnb = std::max(maxnb, nb_of(j1, j2, j, best));
-                if (nw_row[best] >= maxnb) break;
-                nw_row[best]++;
-                used++;
-            }
-            int w = 0;
-            for (int r = 0; r < R; r++)
-                for (int k = 0; k < nw_row[r]; k++, w++) {
-                    lmb[j][w] = (unsigned char)r;
-                    lo[j][w] = (unsigned char)k;
-                    lst[j][w] = (unsigned char)nw_row[r];
+                    cost[mb] += (double)nb_of(j1, j2, j, mb) * (terms + j1 + j2 + 2);
                 }
+        static_assert(TJMAX / 2 + 1 <= YI_WARPS, "a warp for every row");
+        std::vector<int> nw_row(R, 1);
+        for (int used = R; used < YI_WARPS; used++) {
+            int best = 0;
+            for (int r = 1; r < R; r++)
+                if (cost[r] / nw_row[r] > cost[best] / nw_row[best]) best = r;
+            // splitting a row beyond its largest item count buys nothing
+            int maxnb = 0;
+            for (int j1 = 0; j1 <= tj; j1++)
+                for (int j2 = 0; j2 <= j1; j2++)
+                    if (coupling_ok(j1, j2, j)) maxnb = std::max(maxnb, nb_of(j1, j2, j, best));
+            if (nw_row[best] >= maxnb) break;
+            nw_row[best]++;
         }
-        return 0;
-    };
-    if (assign(YI_WARPS, m.yd.lay_mb, m.yd.lay_o, m.yd.lay_st)) {
-        set_error("Y-kernel warp assignment failed");
-        return -1;
+        int w = 0;
+        for (int r = 0; r < R; r++)
+            for (int k = 0; k < nw_row[r]; k++, w++) {
+                m.yl.mb[j][w] = (unsigned char)r;
+                m.yl.o[j][w] = (unsigned char)k;
+                m.yl.st[j][w] = (unsigned char)nw_row[r];
+            }
     }
-    memcpy(m.yq.lay_mb, m.yd.lay_mb, sizeof(m.yd.lay_mb));
-    memcpy(m.yq.lay_o, m.yd.lay_o, sizeof(m.yd.lay_o));
-    memcpy(m.yq.lay_st, m.yd.lay_st, sizeof(m.yd.lay_st));
-
     return 0;
 }
 

@@ -34,30 +34,31 @@ struct SnapGeom {
     int switchflag;
 };
 
-// Y-kernel parameters (the lay_ tables are those of k_snap_yi).  Lanes are the 32 atoms of a tile.  Output layers j are
-// processed one after another by the whole CTA; within a layer every warp walks
-// the same sequence of (j1, j2) couplings, so the code in flight is one
-// coupling's few kilobytes and stays in the instruction cache.  Each warp owns
-// one output row mb of the layer and a residue class of the row-pair index ib,
-// accumulates its share of that row in registers across all couplings, and the
-// warps' partial rows are summed once per layer through shared memory.
-constexpr int YI_MAXW = 24;
+// parameters of the Y kernels
 template <typename T>
 struct YParams {
     T betaY[NTRI];          // beta' of each coupling triple (bnorm 1/(j+1) folded in)
     double e0;              // beta0 - sum_k beta_k bzero_k
-    // per output layer j and warp w: the row mb the warp accumulates (255: idle)
-    // and the residue / stride of the row-pair index ib it takes in every coupling
-    unsigned char lay_mb[JD][YI_MAXW], lay_o[JD][YI_MAXW], lay_st[JD][YI_MAXW];
     // bispectrum component k whose coefficient each coupling triple carries;
     // with per-atom coefficients G[k][atom], the triple's weight is
     // betaY[tri] * G[kmap[tri]] (betaY then holds the multiplicity factors)
     unsigned char kmap[NTRI];
 };
-// warps per Y CTA: 10 (two per row of the costliest layer; 168 registers; 65 ms
-// at 2M atoms against 70 / 71 / 68 / 68 / 74 ms for 9 / 8 / 11 / 12 / 14 warps;
-// its 146 KB U tile leaves room for one CTA per SM)
+// warps per CTA of k_snap_yi: 10 (two per row of the costliest layer; 168
+// registers; 65 ms at 2M atoms against 70 / 71 / 68 / 68 / 74 ms for 9 / 8 / 11 / 12 /
+// 14 warps; its 146 KB U tile leaves room for one CTA per SM)
 constexpr int YI_WARPS = 10;
+// Work of k_snap_yi and k_snap_yi_me.  Lanes are the 32 atoms of a tile.  Output
+// layers j are processed one after another by the whole CTA; within a layer every
+// warp walks the same sequence of (j1, j2) couplings, so the code in flight is one
+// coupling's few kilobytes and stays in the instruction cache.  Each warp owns
+// one output row mb of the layer (255: idle) and of the row-pair index ib the
+// residue class o modulo st in every coupling, accumulates its share of that row
+// in registers across all couplings, and the warps' partial rows are summed once
+// per layer through shared memory.
+struct YiLayout {
+    unsigned char mb[JD][YI_WARPS], o[JD][YI_WARPS], st[JD][YI_WARPS];
+};
 
 __host__ __device__ constexpr bool coupling_ok(int j1, int j2, int j)
 {
@@ -182,25 +183,24 @@ constexpr int UI_WARPS = 4;
 // With pcw, each pair's cutoff and neighbour weight come from pcw[p]; with
 // iblk, atom i is row i % iblk of element block i / iblk of the reference's
 // [block][k][iblk] layout (chemflag U, cpuSnap4.cpp:59-61).
-template <typename T, int TJ>
+template <int TJ>
 __global__ void __launch_bounds__(UI_WARPS * 32)
 k_snap_ui(const int *__restrict__ poff, const double4 *__restrict__ prij, int natoms, SnapGeom gp,
           double *__restrict__ Uref_r, double *__restrict__ Uref_i, const double2 *__restrict__ pcw = nullptr,
           int iblk = 0)
 {
-    typedef typename cplx<T>::type T2;
     constexpr int NU = idxu_count(TJ);
     constexpr int SROW = TJ + 1;
     extern __shared__ __align__(16) unsigned char smraw[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    T2 *acc = reinterpret_cast<T2 *>(smraw) + wib * (NU + 32 * SROW);
-    T2 *stage = acc + NU;
+    double2 *acc = reinterpret_cast<double2 *>(smraw) + wib * (NU + 32 * SROW);
+    double2 *stage = acc + NU;
     const int nwarps = gridDim.x * UI_WARPS;
     for (int i = blockIdx.x * UI_WARPS + wib; i < natoms; i += nwarps) {
-        for (int k = lane; k < NU; k += 32) acc[k] = T2{T(0), T(0)};
+        for (int k = lane; k < NU; k += 32) acc[k] = double2{0.0, 0.0};
         __syncwarp();
         const int p0 = poff[i], p1 = poff[i + 1];
-        T ssum = T(0);
+        double ssum = 0.0;
         for (int base = p0; base < p1; base += 32) {
             const int p = base + lane;
             const bool act = p < p1;
@@ -214,23 +214,23 @@ k_snap_ui(const int *__restrict__ poff, const double4 *__restrict__ prij, int na
             } else {
                 pair_geometry<false>(g, r.x, r.y, r.z, gp);
             }
-            const T sf = act ? (T)g.sfac : T(0);
+            const double sf = act ? g.sfac : 0.0;
             ssum += sf;
-            auto emit = [&](int j, int mb, const T *pr, const T *pi) {
+            auto emit = [&](int j, int mb, const double *pr, const double *pi) {
 #pragma unroll
-                for (int ma = 0; ma <= j; ma++) stage[lane * SROW + ma] = T2{sf * pr[ma], sf * pi[ma]};
+                for (int ma = 0; ma <= j; ma++) stage[lane * SROW + ma] = double2{sf * pr[ma], sf * pi[ma]};
                 __syncwarp();
                 if (lane < 2 * (j + 1)) {
                     const int ma = lane >> 1, c = lane & 1;
-                    const T *col = reinterpret_cast<const T *>(stage + ma) + c;
-                    T s = T(0);
+                    const double *col = reinterpret_cast<const double *>(stage + ma) + c;
+                    double s = 0.0;
                     for (int l = 0; l < nact; l++) s += col[l * SROW * 2];
-                    T *dst = reinterpret_cast<T *>(acc + idxu_block(j) + (j + 1) * mb + ma) + c;
+                    double *dst = reinterpret_cast<double *>(acc + idxu_block(j) + (j + 1) * mb + ma) + c;
                     *dst += s;
                 }
                 __syncwarp();
             };
-            u_rows<T, TJ>((T)g.ar, (T)g.ai, (T)g.br, (T)g.bi, emit);
+            u_rows<double, TJ>(g.ar, g.ai, g.br, g.bi, emit);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, o);
@@ -243,8 +243,8 @@ k_snap_ui(const int *__restrict__ poff, const double4 *__restrict__ prij, int na
             while (idxu_block(j + 1) <= k) j++;
             const int mb = (k - idxu_block(j)) / (j + 1);
             if (2 * mb <= j) {
-                Uref_r[base + (size_t)k * nrow] += (double)acc[k].x;
-                Uref_i[base + (size_t)k * nrow] += (double)acc[k].y;
+                Uref_r[base + (size_t)k * nrow] += acc[k].x;
+                Uref_i[base + (size_t)k * nrow] += acc[k].y;
             }
         }
         __syncwarp();
@@ -408,13 +408,14 @@ __device__ __forceinline__ void z_layer(const int mb, const int o, const int st,
 template <int TJ, bool PA, int J>
 __device__ __forceinline__ void y_layer(const double2 *__restrict__ Us, double2 *__restrict__ red,
                                         double2 *__restrict__ dst, const int lane, const int w,
-                                        const YParams<double> &P, const double *__restrict__ Gs, double &e)
+                                        const YParams<double> &P, const YiLayout &L, const double *__restrict__ Gs,
+                                        double &e)
 {
-    const int mb = P.lay_mb[J][w];
+    const int mb = L.mb[J][w];
     if (mb != 255) {
         YRow<double> acc;
         acc.zero();
-        z_layer<TJ, PA, J, 0, 0>(mb, P.lay_o[J][w], P.lay_st[J][w], Us, lane, P, Gs, acc);
+        z_layer<TJ, PA, J, 0, 0>(mb, L.o[J][w], L.st[J][w], Us, lane, P, Gs, acc);
 #pragma unroll
         for (int ma = 0; ma <= J; ma++) red[(w * JD + ma) * 32 + lane] = acc.get(ma);
     }
@@ -425,7 +426,7 @@ __device__ __forceinline__ void y_layer(const double2 *__restrict__ Us, double2 
         double yr = 0.0, yi = 0.0;
 #pragma unroll
         for (int v = 0; v < YI_WARPS; v++)
-            if (P.lay_mb[J][v] == rmb) {
+            if (L.mb[J][v] == rmb) {
                 const double2 t = red[(v * JD + ma) * 32 + lane];
                 yr += t.x; yi += t.y;
             }
@@ -442,11 +443,12 @@ __device__ __forceinline__ void y_layer(const double2 *__restrict__ Us, double2 
 template <int TJ, bool PA, int J>
 __device__ __forceinline__ void y_all(const double2 *__restrict__ Us, double2 *__restrict__ red,
                                       double2 *__restrict__ dst, const int lane, const int w,
-                                      const YParams<double> &P, const double *__restrict__ Gs, double &e)
+                                      const YParams<double> &P, const YiLayout &L, const double *__restrict__ Gs,
+                                      double &e)
 {
     if constexpr (J >= 0) {
-        y_layer<TJ, PA, J>(Us, red, dst, lane, w, P, Gs, e);
-        y_all<TJ, PA, J - 1>(Us, red, dst, lane, w, P, Gs, e);
+        y_layer<TJ, PA, J>(Us, red, dst, lane, w, P, L, Gs, e);
+        y_all<TJ, PA, J - 1>(Us, red, dst, lane, w, P, L, Gs, e);
     }
 }
 
@@ -474,7 +476,7 @@ constexpr size_t yi_smem_bytes()
 template <int TJ, bool PA>
 __global__ void __launch_bounds__(YI_WARPS * 32, 1)
 k_snap_yi(const double2 *__restrict__ Ut, int natoms, const __grid_constant__ YParams<double> P,
-          double2 *__restrict__ Y, double *__restrict__ eatom, const double *__restrict__ G)
+          const __grid_constant__ YiLayout L, double2 *__restrict__ Y, double *__restrict__ eatom, const double *__restrict__ G)
 {
     constexpr int NW = YI_WARPS;
     constexpr int NU = idxu_count(TJ);
@@ -498,7 +500,7 @@ k_snap_yi(const double2 *__restrict__ Ut, int natoms, const __grid_constant__ YP
         }
         __syncthreads();
         double e = 0.0;
-        y_all<TJ, PA, TJ>(Us, red, Y + (size_t)tile * NYH * 32, lane, w, P, Gs, e);
+        y_all<TJ, PA, TJ>(Us, red, Y + (size_t)tile * NYH * 32, lane, w, P, L, Gs, e);
         if constexpr (PA) {
             __syncthreads();
             continue;
@@ -692,20 +694,20 @@ __device__ __forceinline__ void z_layer_me(const int mb, const int o, const int 
 template <int TJ, int NW, int J>
 __device__ __forceinline__ void y_all_me(const double2 *__restrict__ Ut, const int tile, double2 *__restrict__ red,
                                          double2 *__restrict__ Y, const int lane, const int w,
-                                         const YParams<double> &P, const MeArgs &A, const double *__restrict__ cl,
-                                         const int cs)
+                                         const YParams<double> &P, const YiLayout &L, const MeArgs &A,
+                                         const double *__restrict__ cl, const int cs)
 {
     if constexpr (J >= 0) {
         constexpr int NU = idxu_count(TJ), NYH = yh_count(TJ);
         const int nb = A.nblk;
-        const int mb = P.lay_mb[J][w];
+        const int mb = L.mb[J][w];
         for (int e3 = 0; e3 < nb; e3++) {
             if (mb != 255) {
                 YRow<double> acc;
                 acc.zero();
                 for (int e1 = 0; e1 < nb; e1++)
                     for (int e2 = 0; e2 < nb; e2++)
-                        z_layer_me<TJ, J, 0, 0>(mb, P.lay_o[J][w], P.lay_st[J][w],
+                        z_layer_me<TJ, J, 0, 0>(mb, L.o[J][w], L.st[J][w],
                                                 Ut + ((size_t)e1 * A.ntiles + tile) * NU * 32,
                                                 Ut + ((size_t)e2 * A.ntiles + tile) * NU * 32, lane, P, cl, cs,
                                                 (e1 * nb + e2) * nb + e3, (e3 * nb + e2) * nb + e1,
@@ -721,7 +723,7 @@ __device__ __forceinline__ void y_all_me(const double2 *__restrict__ Ut, const i
                 double yr = 0.0, yi = 0.0;
 #pragma unroll
                 for (int v = 0; v < NW; v++)
-                    if (P.lay_mb[J][v] == rmb) {
+                    if (L.mb[J][v] == rmb) {
                         const double2 t = red[(v * JD + ma) * 32 + lane];
                         yr += t.x; yi += t.y;
                     }
@@ -729,7 +731,7 @@ __device__ __forceinline__ void y_all_me(const double2 *__restrict__ Ut, const i
             }
             __syncthreads();
         }
-        y_all_me<TJ, NW, J - 1>(Ut, tile, red, Y, lane, w, P, A, cl, cs);
+        y_all_me<TJ, NW, J - 1>(Ut, tile, red, Y, lane, w, P, L, A, cl, cs);
     }
 }
 
@@ -742,7 +744,7 @@ constexpr size_t yi_me_smem_bytes()
 template <int TJ>
 __global__ void __launch_bounds__(YI_WARPS * 32, 1)
 k_snap_yi_me(const double2 *__restrict__ Ut, int natoms, const __grid_constant__ YParams<double> P,
-             const __grid_constant__ MeArgs A, double2 *__restrict__ Y)
+             const __grid_constant__ YiLayout L, const __grid_constant__ MeArgs A, double2 *__restrict__ Y)
 {
     constexpr int NW = YI_WARPS;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -751,10 +753,10 @@ k_snap_yi_me(const double2 *__restrict__ Ut, int natoms, const __grid_constant__
     for (int tile = blockIdx.x; tile < A.ntiles; tile += gridDim.x) {
         const int atom = tile * 32 + lane;
         if (A.pa) {
-            y_all_me<TJ, NW, TJ>(Ut, tile, red, Y, lane, w, P, A, A.coeff + (atom < natoms ? atom : 0), natoms);
+            y_all_me<TJ, NW, TJ>(Ut, tile, red, Y, lane, w, P, L, A, A.coeff + (atom < natoms ? atom : 0), natoms);
         } else {
             const int ie = atom < natoms ? A.elem[atom] : 0;
-            y_all_me<TJ, NW, TJ>(Ut, tile, red, Y, lane, w, P, A, A.coeff + (size_t)ie * A.ncoeffall + 1, 1);
+            y_all_me<TJ, NW, TJ>(Ut, tile, red, Y, lane, w, P, L, A, A.coeff + (size_t)ie * A.ncoeffall + 1, 1);
         }
     }
 }

@@ -214,14 +214,9 @@ __device__ __forceinline__ void ur_dispatch(const int job, const int *__restrict
 // run close together and its pairs come from L2 once.  SPL lanes share an
 // atom's pairs (few atoms); the pad lanes of the last tile write empty sums.
 constexpr int UR_WARPS = 4;
-#ifndef UR_MINB_D
-#define UR_MINB_D 3
-#endif
-#ifndef UR_MINB_F
-#define UR_MINB_F 4
-#endif
+template <typename T> __host__ __device__ constexpr int ur_min_ctas() { return sizeof(T) == 8 ? 3 : 4; }
 template <typename T, int TJ, int SPL>
-__global__ void __launch_bounds__(UR_WARPS * 32, sizeof(T) == 8 ? UR_MINB_D : UR_MINB_F)
+__global__ void __launch_bounds__(UR_WARPS * 32, ur_min_ctas<T>())
 k_snap_ur(const int *__restrict__ poff, const double4 *__restrict__ prij, const double4 *__restrict__ pab, int natoms,
           typename cplx<T>::type *__restrict__ Ut, const int *__restrict__ welem, int ipad)
 {
