@@ -537,7 +537,6 @@ int launch_y_part(const YParams<T> &yp, ForcePath &fp, int inum, int t0, int nt,
         k_snap_y<T, TJ, PA><<<ctas, NT, sm, s>>>(U, atoms, yp, plans[0], 1, Y, n, eatom, nullptr, G, inum);
         return 0;
     }
-    if (fp.Ypart.ensure(sizeof(T2) * n * ng) || fp.esum.ensure(sizeof(double) * (size_t)atoms * ng)) return -1;
     k_snap_y<T, TJ, PA><<<ctas * ng, NT, sm, s>>>(U, atoms, yp, plans[ng - 1], ng, fp.Ypart.as<T2>(), n, eatom,
                                                    fp.esum.as<double>(), G, inum);
     k_y_sum<T2><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(fp.Ypart.as<T2>(), n, ng, Y, fp.esum.as<double>(), atoms,
@@ -557,6 +556,12 @@ int launch_y(const YParams<T> &yp, ForcePath &fp, int inum, double *eatom, const
     int per_sm = 0;
     if (kernel_setup((const void *)k_snap_y<T, TJ, PA>, NT, y_smem_bytes<T, TJ, PA>(), &per_sm, "k_snap_y")) return -1;
     const int nt = (inum + 31) / 32, wave = num_sms() * per_sm, ctas = (nt + NTI - 1) / NTI, rem = ctas % wave;
+    // The groups' parts fill at most a wave's tiles (12 MB).  The room is taken at
+    // the first call of any size: a smaller system can need more of it than a
+    // larger one, and a buffer must not grow while a call is captured.
+    if (TJ > 4 && (fp.Ypart.ensure(sizeof(typename cplx<T>::type) * wave * NTI * yh_count(TJ) * 32) ||
+                   fp.esum.ensure(sizeof(double) * wave * NTI * 32)))
+        return -1;
     if (TJ > 4 && ctas > wave && ctas < 16 * wave && rem > 0 && 2 * rem <= wave) {
         const int t0 = (ctas - rem) * NTI;
         if (launch_y_part<T, TJ, PA>(yp, fp, inum, 0, t0, wave, eatom, G, s)) return -1;
