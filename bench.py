@@ -59,24 +59,31 @@ SAMPLE_CELLS = (20, 20, 20)        # CPU-baseline sample: 16,000 atoms
 
 
 
-def fr_flops_per_pair(tj):
-    """FLOPs of the reverse-mode dE/dr of one pair (an FMA counts 2).
+# jobs of the one-sweep dE/dr at 2J = 8: column, its first and last layer, and
+# whether the job also takes the middle row of the top layer
+FC_JOBS = ((3, 6, 8, 1), (0, 7, 8, 0), (1, 7, 8, 0), (2, 7, 8, 0), (0, 0, 6, 0), (1, 2, 6, 0), (2, 4, 6, 0))
 
-    Forward row step of layer J: 2 end entries x 8 + (J-1) inner x 18.
-    Adjoint step of layer J: gradient 10 per coupling term (2J of them),
-    parent adjoint 18 per entry (J), weighted Y 2 per entry of layer J-1.
-    Rows recomputed: the seed sweep (layers 2mb, 2mb+1 of columns
-    mb < tj/2) and each column's layers below tj.
+
+def fc_flops_per_pair():
+    """FLOPs of the one-sweep dE/dr of one pair at 2J = 8, the form that runs at
+    this size, with the rows that its jobs compute again (an FMA counts 2).
+
+    A row step of layer J is two end entries of 6 and J - 1 inner ones of 14;
+    each entry of a job's rows feeds four sums: F, Gx and Gy 4 each, Gz 5 (none
+    at a middle row's centre).
     """
     def fwd(j):
-        return 16 + 18 * (j - 1)
+        return 12 + 14 * (j - 1) if j else 0
+
+    def dot(j, n):
+        return sum(12 + (5 if 2 * m != j else 0) for m in range(n))
     fl = 0
-    for mb in range(tj // 2):                       # seed sweep
-        fl += sum(fwd(j) for j in ((1,) if mb == 0 else (2 * mb, 2 * mb + 1)))
-    for mb in range(tj // 2 + 1):
-        j0 = 1 if mb == 0 else 2 * mb
-        fl += sum(fwd(j) for j in range(j0, tj))     # column recompute
-        fl += sum(10 * 2 * j + 18 * j + 2 * j for j in range(j0, tj + 1))   # adjoint
+    for mb, lo, hi, top in FC_JOBS:
+        fl += sum(fwd(2 * c) + fwd(2 * c + 1) for c in range(mb))          # the column's seed
+        fl += sum(fwd(j) for j in range(2 * mb, hi + 1))
+        fl += sum(dot(j, mb + 1 if 2 * mb == j else j + 1) for j in range(lo, hi + 1))
+        if top:
+            fl += fwd(TWOJ) + dot(TWOJ, TWOJ // 2 + 1)
     return fl
 
 
@@ -84,10 +91,10 @@ def fr_flops_per_pair(tj):
 # two U entries once: 14,880 complex products, 39,977 of them times a real
 # coefficient added to a layer's sum, 8,712 of those sums scaled and added to Y)
 # and the energy's 155 x 4; U 154 half-plane elements x 22 per pair (the
-# reference's recursion), dE/dr as implemented (reverse mode)
+# reference's recursion), dE/dr as implemented
 FLOP_Y_PER_ATOM = 14880 * 6 + 39977 * 4 + 8712 * 4 + 155 * 4
 FLOP_U_PER_PAIR = 154 * 22
-FLOP_F_PER_PAIR = fr_flops_per_pair(8)
+FLOP_F_PER_PAIR = fc_flops_per_pair()
 
 
 def dist_env():
@@ -294,7 +301,13 @@ def run_reference(args):
     ws, rank, _ = dist_env()
     if rank != 0:
         return
-    s = CpuSample()
+    try:
+        s = CpuSample()
+    except (subprocess.CalledProcessError, OSError) as ex:
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "MDP's CPU library could not be built from its sources: " + str(ex)[:150]}),
+              flush=True)
+        return
     for _ in range(args.warmup):
         s.step()
     el = sum(s.step() for _ in range(args.steps))
